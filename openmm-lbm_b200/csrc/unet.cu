@@ -1,11 +1,13 @@
 // Tensor-core 3x3x3 convolutions of the learned warm start (include/lbm_b200_warmstart.h), written for sm_100a:
 //
-//  convForwardKernel    y[voxel][cout] = sum_k A[voxel][k] W[cout][k], k = tap*cin + ci, A the implicit im2col of x
-//                       (zero padding); one CTA per 128 voxels, all cout in one N tile (<= 256)
+//  convSliceKernel      y[voxel][cout] = sum_k A[voxel][k] W[cout][k], k = tap*cin + ci, A the implicit im2col of x
+//                       (zero padding), read in place from slices of x in shared memory
+//  convForwardKernel    the same for the channel counts that the slices do not serve: A gathered per 128 voxels, all
+//                       cout in one N tile (<= 256)
 //  convWeightGradKernel dW[cout][k] = sum_voxels dy[voxel][cout] A[voxel][k]; CTAs over (cout tile, k tile, voxel
 //                       split), the K dimension of the GEMM being the voxels; results added with FP32 atomics
 //
-// The GEMM core: 128 x N tiles, K in stages of 64 BF16 (one 128-byte row).  All 128 threads gather a stage into
+// The GEMM core of the gathering kernels: 128 x N tiles, K in stages of 64 BF16 (one 128-byte row).  All 128 threads gather a stage into
 // shared memory in the canonical K-major layout with the 128-byte swizzle (8-row atoms of 128-byte rows, the 16-byte
 // chunk index XOR the row within the atom), make it visible to the tensor core's proxy, and one thread issues four
 // tcgen05.mma (K = 16 each, BF16 x BF16 -> FP32 in tensor memory) and commits them to an mbarrier that every
@@ -20,6 +22,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <string>
+#include <type_traits>
 
 namespace {
 
@@ -95,8 +98,8 @@ __device__ __forceinline__ void tmemLoad8(uint32_t addr, float v[8]) {
         v[i] = __uint_as_float(r[i]);
 }
 
-__device__ __forceinline__ uint32_t tmemColumns(int n) {
-    return n <= 32 ? 32u : (n <= 64 ? 64u : (n <= 128 ? 128u : 256u));
+__host__ __device__ inline uint32_t tmemColumns(int n) {
+    return n <= 32 ? 32u : (n <= 64 ? 64u : (n <= 128 ? 128u : (n <= 256 ? 256u : 512u)));
 }
 
 // Setup common to both kernels: 1024-byte aligned tiles, tensor memory of `ncols` columns (warp 0), the mbarrier.
@@ -160,6 +163,476 @@ __device__ __forceinline__ bool runStage(const Stage& st, uint32_t idesc, int st
 __device__ __forceinline__ void drainStage(const Stage& st, int stage) {
     waitParity(st.mbar, (uint32_t) (stage & 1), kSpinLimit);
     __syncthreads();
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// The forward convolution from slices of the input held in shared memory.
+//
+// A CTA owns a column of 8 x 16 voxels (x, y) of one volume and `nTile` output channels, and marches over `zLen`
+// planes: plane z of the output is one M = 128 tile (row = 8 y + x) with an accumulator of its own in tensor memory.
+// Each input slice (10 x 18 voxels with the halo, zero outside the volume) is copied once into a ring of slots, laid
+// out as [8-channel group][voxel] x 16 bytes: 8 x-neighbours are a core matrix of the unswizzled K-major layout, the
+// y rows are 160 bytes apart (stride offset), the channel groups kPlane bytes (leading offset), and a tap is nothing
+// but another start address in the slot.  Slice s takes part in the planes s - 1 (taps dz = +1), s and s + 1
+// (dz = -1), so every plane receives its products in the order (tap, channel), 16 channels per tcgen05.mma: the order
+// of the gathering kernel below, and its results bit for bit.
+//
+// Warps 0-3 read the accumulators (bias, ReLU, BF16 stores), warp 4 issues the MMAs, warps 5-8 copy slices and
+// weight tiles with cp.async and hand them over through mbarriers.  The weights of one tap are a tile of
+// [8-channel group][output channel] x 16 bytes; all 27 stay resident when they fit (wSlots = 27), otherwise they
+// stream through a ring of wSlots tiles.
+//
+// Bound: an MMA of M = 128 and N <= 64 reads 4 KB of A (36 wavefronts of shared memory with 16 channels of B) and holds
+// the tensor core for 52 cycles, 41 us for 16 -> 16 channels on two 64 x 64 x 128 volumes.  Measured there: 47 us
+// (229 us with the gathering kernel, whose threads fetch every voxel 27 times and wait for each stage's MMAs); 48 -> 16
+// 124 us (880), 32 -> 32 at 32 x 32 x 64 30 us (84), 160 -> 160 at 8 x 8 x 16 38 us (307).  With one thread issuing from
+// divergent code the same layer took 82 us (its operands went through general registers, 140-200 cycles per MMA), and
+// with the planes' MMAs interleaved tap by tap 111 us (a branch per MMA).
+// ---------------------------------------------------------------------------------------------------------------
+
+constexpr int kTileX = 8, kTileY = 16, kHaloX = kTileX + 2, kHaloY = kTileY + 2;
+constexpr int kSliceVoxels = kHaloX*kHaloY;
+constexpr int kPlane = kSliceVoxels*16 + 16;   // bytes per channel group; + 16 spreads the groups over the banks
+constexpr int kMaxSlots = 24, kMaxAcc = 8, kTaps = 27;
+constexpr int kEpilogueThreads = 128, kProducersResident = 128, kProducersStreamed = 256;
+constexpr int kZeroZone = 15*kHaloX*16 + 128;  // 16 core matrices at the stride of the y rows, all zero (cin = 8)
+
+struct SliceParams {
+    const __nv_bfloat16* x;
+    const __nv_bfloat16* w;
+    const float* bias;
+    __nv_bfloat16* y;
+    int batch, D, H, W, cin, cout, relu;
+    int nTile, zLen, slots, wSlots, accSlots;
+    int colsX, colsY, zBlocks, nBlocks, items;
+};
+
+struct SliceBarriers {
+    uint64_t full[kMaxSlots], empty[kMaxSlots], wFull[kTaps], wEmpty[kTaps], accFull[kMaxAcc], accEmpty[kMaxAcc], drain;
+    uint32_t tmem;
+    int stop;
+};
+
+__host__ __device__ inline int sliceBytes(int cin) { return (cin/8)*kPlane; }
+// A weight tile: nTile channels of a group at 16 bytes, + 16 per group to spread the groups over the banks.
+__host__ __device__ inline int weightGroupBytes(int nTile) { return nTile*16 + 16; }
+__host__ __device__ inline int weightTileBytes(int cin, int nTile) { return (cin/8)*weightGroupBytes(nTile); }
+__host__ __device__ inline size_t sliceSmemBytes(int cin, int nTile, int slots, int wSlots) {
+    // The single-group layout pairs taps: a 28th tile of zeros and a zero slice stand in for the tap after the last.
+    return sizeof(SliceBarriers) + 128 + (size_t) slots*sliceBytes(cin) + (size_t) wSlots*weightTileBytes(cin, nTile)
+         + (cin == 8 ? kZeroZone + weightTileBytes(cin, nTile) : 0);
+}
+
+struct SliceItem {
+    int n, x0, y0, z0, zc, co0;    // volume, origin of the column, first plane, planes, first output channel
+};
+
+__device__ __forceinline__ SliceItem sliceItem(const SliceParams& p, int item) {
+    SliceItem t;
+    int r = item;
+    const int cx = r%p.colsX; r /= p.colsX;
+    const int cy = r%p.colsY; r /= p.colsY;
+    const int zb = r%p.zBlocks; r /= p.zBlocks;
+    const int nb = r%p.nBlocks;
+    t.n = r/p.nBlocks;
+    t.x0 = cx*kTileX;
+    t.y0 = cy*kTileY;
+    t.z0 = zb*p.zLen;
+    t.zc = min(p.zLen, p.D - t.z0);
+    t.co0 = nb*p.nTile;
+    return t;
+}
+
+__device__ __forceinline__ void arrive(uint32_t mbar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(mbar) : "memory");
+}
+
+// A bounded wait that also ends when another role of the CTA has given up; a wait that runs out makes all give up.
+__device__ __forceinline__ bool waitOrStop(uint32_t mbar, uint32_t parity, long long limit, volatile int* stop) {
+    for (long long i = 0; i < limit; i++) {
+        uint32_t done;
+        asm volatile("{\n\t.reg .pred P1;\n\tmbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
+                     "selp.b32 %0, 1, 0, P1;\n\t}" : "=r"(done) : "r"(mbar), "r"(parity) : "memory");
+        if (done)
+            return true;
+        if (*stop)
+            return false;
+    }
+    *stop = 1;
+    return false;
+}
+
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+
+// The 16-byte pieces of a copy that thread `first` of `step` threads takes, channel group fastest, without divisions in
+// the loop: (g, v) is group g of voxel (or output channel) v.
+struct Pieces {
+    int g, v, groups, stepG, stepV;
+    __device__ __forceinline__ Pieces(int first, int step, int groups)
+            : g(first%groups), v(first/groups), groups(groups), stepG(step%groups), stepV(step/groups) {}
+    __device__ __forceinline__ void next(int& pg, int& pv) const {
+        pg += stepG;
+        const bool carry = pg >= groups;
+        pg -= carry ? groups : 0;
+        pv += stepV + (carry ? 1 : 0);
+    }
+};
+
+// The copies of one producer thread: groups are handed over (proxy fence, arrive) when they have landed, at most kLag
+// of them in flight; a producer that has to wait for a free slot hands over all of them first, since the consumer may
+// be waiting for exactly those.
+struct CopyQueue {
+    static constexpr int kLag = 3;
+    uint32_t bars[kLag];
+    int count = 0;
+    __device__ __forceinline__ void pop() {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        arrive(bars[0]);
+        for (int i = 1; i < kLag; i++)
+            bars[i-1] = bars[i];
+        count--;
+    }
+    __device__ __forceinline__ void push(uint32_t bar) {
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        for (int i = 0; i < kLag; i++)
+            if (i == count)
+                bars[i] = bar;
+        count++;
+        if (count == kLag) {
+            asm volatile("cp.async.wait_group %0;" :: "n"(kLag - 1) : "memory");
+            pop();
+        }
+    }
+    __device__ __forceinline__ void flush() {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        while (count > 0)
+            pop();
+    }
+    // Waits until `bar` has completed the phase `parity`.
+    __device__ __forceinline__ bool waitFree(uint32_t bar, uint32_t parity, long long limit, volatile int* stop) {
+        if (count > 0) {
+            uint32_t done;
+            asm volatile("{\n\t.reg .pred P1;\n\tmbarrier.test_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
+                         "selp.b32 %0, 1, 0, P1;\n\t}" : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+            if (!done)
+                flush();
+        }
+        return waitOrStop(bar, parity, limit, stop);
+    }
+};
+
+// The MMA and the commit as a converged warp issues them: the whole warp computes the (uniform) operands, which keeps
+// them in uniform registers, and one elected lane issues.
+__device__ __forceinline__ void mmaElected(uint32_t tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\telect.sync _|q, 0xffffffff;\n\t"
+                 "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+                 :: "r"(tmem), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void commitElected(uint32_t mbar) {
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+                 "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" :: "r"(mbar) : "memory");
+}
+// waitOrStop by a whole warp, with one answer for all lanes.
+__device__ __forceinline__ bool warpWait(uint32_t mbar, uint32_t parity, long long limit, volatile int* stop) {
+    return __all_sync(0xffffffffu, waitOrStop(mbar, parity, limit, stop));
+}
+
+// A matrix descriptor from its words: the low one holds the start address and the leading offset, the high one the
+// stride offset and the version (unswizzled layouts).
+__device__ __forceinline__ uint64_t join(uint32_t low, uint32_t high) {
+    return (uint64_t) high << 32 | low;
+}
+
+// How a CTA holds its weights: all 27 taps resident, streamed tap by tap, or resident with one channel group per tap
+// (cin = 8), where an MMA takes two taps.
+enum { kResident, kStreamed, kSingleGroup };
+
+template <int MODE>
+constexpr int sliceThreads = kEpilogueThreads + 32 + (MODE == kStreamed ? kProducersStreamed : kProducersResident);
+
+template <int MODE>
+__global__ void __launch_bounds__(sliceThreads<MODE>)
+convSliceKernel(const SliceParams p) {
+    extern __shared__ __align__(128) uint8_t smemRaw[];
+    SliceBarriers* bars = reinterpret_cast<SliceBarriers*>(smemRaw);
+    const int slotBytes = sliceBytes(p.cin), tileBytes = weightTileBytes(p.cin, p.nTile);
+    const uint32_t ring = (smemAddr(smemRaw) + (uint32_t) sizeof(SliceBarriers) + 127u) & ~127u;
+    const uint32_t zeroZone = ring + (uint32_t) (p.slots*slotBytes);
+    const uint32_t weights = zeroZone + (p.cin == 8 ? kZeroZone : 0);
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid/32, 0), lane = tid%32;
+    const uint32_t ncols = tmemColumns(p.accSlots*p.nTile);
+    volatile int* stop = &bars->stop;
+    constexpr bool resident = MODE != kStreamed;
+    constexpr int producerThreads = sliceThreads<MODE> - kEpilogueThreads - 32;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smemAddr(&bars->tmem)), "r"(ncols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    if (tid == 32) {
+        auto init = [](uint64_t* b, int count) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smemAddr(b)), "r"(count) : "memory");
+        };
+        for (int i = 0; i < p.slots; i++) {
+            init(&bars->full[i], producerThreads);
+            init(&bars->empty[i], 1);
+        }
+        for (int i = 0; i < p.wSlots; i++) {
+            init(&bars->wFull[i], resident ? producerThreads : 32);
+            init(&bars->wEmpty[i], 1);
+        }
+        for (int i = 0; i < p.accSlots; i++) {
+            init(&bars->accFull[i], 1);
+            init(&bars->accEmpty[i], kEpilogueThreads);
+        }
+        init(&bars->drain, 1);
+        bars->stop = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (p.cin == 8) {
+        for (int i = tid; i < kZeroZone/16; i += sliceThreads<MODE>)
+            *reinterpret_cast<uint4*>(smemRaw + (zeroZone - smemAddr(smemRaw)) + 16*i) = make_uint4(0, 0, 0, 0);
+        for (int i = tid; i < tileBytes/16; i += sliceThreads<MODE>)
+            *reinterpret_cast<uint4*>(smemRaw + (weights - smemAddr(smemRaw)) + kTaps*tileBytes + 16*i) = make_uint4(0, 0, 0, 0);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    fenceBeforeSync();
+    __syncthreads();
+    fenceAfterSync();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, bars->tmem, 0);
+    const long long limit = convWaitPolls;
+    const int groups = p.cin/8;
+
+    if (warp >= 5) {
+        // ---- producers: slices in the order of the planes (all warps share a slice), and the weight tiles in the order
+        // of their use (one warp each in turn when streamed, so that the tiles' latencies overlap) ----
+        const int t = tid - (kEpilogueThreads + 32), producers = producerThreads;
+        // At most wSlots warps: one that is further ahead would take a slot's phase for the one two before it.
+        const int pw = warp - 5, warps = min(producers/32, p.wSlots);
+        CopyQueue queue;
+        const Pieces bySlice(t, producers, groups), byTile(lane, 32, groups), byAll(t, producers, groups);
+        const int groupW = weightGroupBytes(p.nTile);
+        int tile = 0, slot = 0, wSlot = 0;
+        uint32_t slotPhase = 1, wPhase = 1;        // a free slot's barrier has completed the phase before its first
+        bool ok = true;
+        auto copyTile = [&](const Pieces& pieces, int at, int tap, int co0) {
+            const uint32_t base = weights + (uint32_t) (at*tileBytes);
+            const __nv_bfloat16* src = p.w + ((size_t) co0*kTaps + tap)*p.cin;
+            for (int g = pieces.g, n = pieces.v; n < p.nTile; ) {
+                copy16(base + (uint32_t) (g*groupW + n*16), src + (size_t) n*kTaps*p.cin + 8*g, true);
+                pieces.next(g, n);
+            }
+        };
+        for (int item = blockIdx.x; item < p.items && ok; item += gridDim.x) {
+            const SliceItem it = sliceItem(p, item);
+            for (int s = 0; s < it.zc + 2 && ok; s++) {
+                const int z = it.z0 + s - 1;
+                ok = queue.waitFree(smemAddr(&bars->empty[slot]), slotPhase, limit, stop);
+                if (!ok)
+                    break;
+                const uint32_t base = ring + (uint32_t) (slot*slotBytes);
+                const bool inside = z >= 0 && z < p.D;
+                const __nv_bfloat16* plane = p.x + ((size_t) it.n*p.D + (inside ? z : 0))*p.H*p.W*p.cin;
+                for (int g = bySlice.g, v = bySlice.v; v < kSliceVoxels; ) {
+                    const int vy = v/kHaloX, yy = it.y0 + vy - 1, xx = it.x0 + (v - vy*kHaloX) - 1;
+                    const bool valid = inside && (unsigned) yy < (unsigned) p.H && (unsigned) xx < (unsigned) p.W;
+                    copy16(base + (uint32_t) (g*kPlane + v*16), plane + (valid ? (yy*p.W + xx)*p.cin + 8*g : 0), valid);
+                    bySlice.next(g, v);
+                }
+                queue.push(smemAddr(&bars->full[slot]));
+                if (++slot == p.slots) {
+                    slot = 0;
+                    slotPhase ^= 1;
+                }
+                for (int dz = 2; dz >= 0 && ok; dz--) {
+                    // Plane z0 + s - dz takes the taps 9 dz .. 9 dz + 8 from this slice; resident tiles come with the
+                    // CTA's first plane.
+                    if (s - dz < 0 || s - dz >= it.zc || (resident && (item != blockIdx.x || s != dz)))
+                        continue;
+                    for (int k = 0; k < 9 && ok; k++) {
+                        if (resident) {
+                            copyTile(byAll, 9*dz + k, 9*dz + k, it.co0);
+                            continue;
+                        }
+                        if (tile++%warps == pw) {
+                            ok = queue.waitFree(smemAddr(&bars->wEmpty[wSlot]), wPhase, limit, stop);
+                            if (!ok)
+                                break;
+                            copyTile(byTile, wSlot, 9*dz + k, it.co0);
+                            queue.push(smemAddr(&bars->wFull[wSlot]));
+                        }
+                        if (++wSlot == p.wSlots) {
+                            wSlot = 0;
+                            wPhase ^= 1;
+                        }
+                    }
+                    if (resident)
+                        queue.push(smemAddr(&bars->wFull[dz]));
+                }
+            }
+        }
+        queue.flush();
+    }
+    else if (warp == 4) {
+        // ---- the MMAs: the instructions between two of them are what a narrow layer waits for, so the taps are
+        // unrolled, a descriptor is its low word plus a constant, and the warp stays converged (uniform registers) ----
+        {
+            const uint32_t idesc = instrDescriptor(p.nTile);
+            const uint32_t groupW = (uint32_t) weightGroupBytes(p.nTile), tileUnits = (uint32_t) tileBytes/16;
+            const uint32_t aHigh = (kHaloX*16 >> 4) | (1u << 14), bHigh = (128 >> 4) | (1u << 14);
+            const uint32_t wLow = (weights >> 4) | ((MODE == kSingleGroup ? (uint32_t) tileBytes : groupW) >> 4 << 16);
+            int plane0 = 0, slot = 0, wSlot = 0;
+            uint32_t slotPhase = 0, wPhase = 0;
+            bool ok = true, issued = false;
+            for (int item = blockIdx.x; item < p.items && ok; item += gridDim.x) {
+                const SliceItem it = sliceItem(p, item);
+                for (int s = 0; s < it.zc + 2 && ok; s++) {
+                    ok = warpWait(smemAddr(&bars->full[slot]), slotPhase, limit, stop);
+                    if (!ok)
+                        break;
+                    const uint32_t base = ring + (uint32_t) (slot*slotBytes);
+                    auto stage = [&](auto dzc) {
+                        constexpr int dz = decltype(dzc)::value;
+                        const int k0 = s - dz;
+                        if (k0 < 0 || k0 >= it.zc || !ok)
+                            return;
+                        const int plane = plane0 + k0, acc = plane%p.accSlots;
+                        const uint32_t d = tmem + (uint32_t) (acc*p.nTile);
+                        if (dz == 0 && plane >= p.accSlots) {
+                            ok = warpWait(smemAddr(&bars->accEmpty[acc]), (uint32_t) ((plane/p.accSlots - 1) & 1), limit, stop);
+                            if (!ok)
+                                return;
+                            fenceAfterSync();
+                        }
+                        if (MODE != kStreamed && item == blockIdx.x && k0 == 0)
+                            ok = warpWait(smemAddr(&bars->wFull[dz]), 0, limit, stop);
+                        if (!ok)
+                            return;
+                        issued = true;
+                        if constexpr (MODE == kSingleGroup) {
+                            // Two taps per MMA, (0,1) (2,3) ... (26, zero): K = 16 is two groups a leading offset apart.
+                            constexpr int first = dz == 0 ? 0 : (dz == 1 ? 8 : 18), count = dz == 0 ? 4 : 5;
+#pragma unroll
+                            for (int i = 0; i < count; i++) {
+                                const int tap = first + 2*i, r = tap%9, r1 = (tap + 1)%9;
+                                const uint32_t here = base - (tap == 8 ? (uint32_t) slotBytes : 0u);
+                                const uint32_t from = here + (uint32_t) ((r/3)*kHaloX + r%3)*16;
+                                const uint32_t to = tap == 26 ? zeroZone : base + (uint32_t) ((r1/3)*kHaloX + r1%3)*16;
+                                mmaElected(d, join((from >> 4) | ((to - from) >> 4 << 16), aHigh),
+                                        join(wLow + (uint32_t) tap*tileUnits, bHigh), idesc, tap > 0 ? 1u : 0u);
+                            }
+                        }
+                        else {
+                            const uint32_t aLow = (base >> 4) | (uint32_t) (kPlane/16) << 16;
+                            uint32_t bLow = wLow + 9*dz*tileUnits;
+#pragma unroll
+                            for (int r = 0; r < 9; r++) {
+                                if constexpr (MODE == kStreamed) {
+                                    ok = ok && warpWait(smemAddr(&bars->wFull[wSlot]), wPhase, limit, stop);
+                                    if (!ok)
+                                        return;
+                                    bLow = wLow + (uint32_t) wSlot*tileUnits;
+                                }
+                                uint32_t a = aLow + (uint32_t) ((r/3)*kHaloX + r%3), b = bLow;
+                                mmaElected(d, join(a, aHigh), join(b, bHigh), idesc, dz > 0 || r > 0 ? 1u : 0u);
+                                for (int g = 2; g < groups; g += 2) {
+                                    a += 2*kPlane/16;
+                                    b += groupW/8;
+                                    mmaElected(d, join(a, aHigh), join(b, bHigh), idesc, 1u);
+                                }
+                                if constexpr (MODE == kStreamed) {
+                                    commitElected(smemAddr(&bars->wEmpty[wSlot]));
+                                    if (++wSlot == p.wSlots) {
+                                        wSlot = 0;
+                                        wPhase ^= 1;
+                                    }
+                                }
+                                else
+                                    bLow += tileUnits;
+                            }
+                        }
+                        if (dz == 2)
+                            commitElected(smemAddr(&bars->accFull[acc]));
+                    };
+                    stage(std::integral_constant<int, 2>());
+                    stage(std::integral_constant<int, 1>());
+                    stage(std::integral_constant<int, 0>());
+                    if (!ok)
+                        break;
+                    // The slice is free once its MMAs are done; with one group the next slice's first pair still reads
+                    // it, so each slice is freed one slice later, the last two of a column together.
+                    if (MODE != kSingleGroup)
+                        commitElected(smemAddr(&bars->empty[slot]));
+                    else {
+                        if (s > 0)
+                            commitElected(smemAddr(&bars->empty[slot - 1]));
+                        if (s == it.zc + 1)
+                            commitElected(smemAddr(&bars->empty[slot]));
+                    }
+                    if (++slot == p.slots) {
+                        slot = 0;
+                        slotPhase ^= 1;
+                    }
+                }
+                plane0 += it.zc;
+            }
+            // The MMAs and arrivals in flight end before the CTA leaves (a role may have given up).
+            if (issued) {
+                commitElected(smemAddr(&bars->drain));
+                waitParity(smemAddr(&bars->drain), 0, kSpinLimit);
+                __syncwarp();
+            }
+        }
+    }
+    else {
+        // ---- epilogue: warp w owns the lanes 32 w .. 32 w + 31 of the accumulators, rows of the tile ----
+        const int row = warp*32 + lane, vx = row%kTileX, vy = row/kTileX;
+        int plane0 = 0;
+        bool ok = true;
+        for (int item = blockIdx.x; item < p.items && ok; item += gridDim.x) {
+            const SliceItem it = sliceItem(p, item);
+            const int xx = it.x0 + vx, yy = it.y0 + vy;
+            const bool store = xx < p.W && yy < p.H;
+            for (int k = 0; k < it.zc; k++) {
+                const int plane = plane0 + k, acc = plane%p.accSlots;
+                ok = waitOrStop(smemAddr(&bars->accFull[acc]), (uint32_t) ((plane/p.accSlots) & 1), limit, stop);
+                if (!ok)
+                    break;
+                fenceAfterSync();
+                const uint32_t d = tmem + ((uint32_t) (warp*32) << 16) + (uint32_t) (acc*p.nTile);
+                __nv_bfloat16* out = p.y + ((((size_t) it.n*p.D + it.z0 + k)*p.H + yy)*p.W + xx)*p.cout + it.co0;
+                for (int col = 0; col < p.nTile; col += 16) {
+                    uint32_t v[16];
+                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
+                                 "%13, %14, %15}, [%16];"
+                                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                                   "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
+                                   "=r"(v[15]) : "r"(d + (uint32_t) col));
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (store) {
+                        __align__(16) __nv_bfloat16 o[16];
+#pragma unroll
+                        for (int i = 0; i < 16; i++) {
+                            const float f = __uint_as_float(v[i]) + (p.bias ? __ldg(p.bias + it.co0 + col + i) : 0.0f);
+                            o[i] = __float2bfloat16_rn(p.relu ? fmaxf(f, 0.0f) : f);
+                        }
+                        reinterpret_cast<uint4*>(out + col)[0] = reinterpret_cast<const uint4*>(o)[0];
+                        reinterpret_cast<uint4*>(out + col)[1] = reinterpret_cast<const uint4*>(o)[1];
+                    }
+                }
+                fenceBeforeSync();
+                arrive(smemAddr(&bars->accEmpty[acc]));
+            }
+            plane0 += it.zc;
+        }
+    }
+    fenceBeforeSync();
+    __syncthreads();
+    if (tid == 0 && bars->stop)
+        atomicExch(&convStatus, (int) LBM_ERR_DEVICE_TIMEOUT);
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(ncols) : "memory");
 }
 
 __global__ void __launch_bounds__(kThreads)
@@ -312,6 +785,78 @@ size_t stageBytes(int rowsB) {
     return 1024 + (size_t) kTileM*128 + (size_t) rowsB*128 + 64;
 }
 
+// The slice kernel's division of a layer: which channels, planes and slots a CTA takes.  false where it does not apply
+// (cin of an odd number of 8-channel groups other than one, whose 16-channel steps straddle taps; slices too wide for
+// two slots in shared memory, above 224-240 channels): the gathering kernel takes those.  Where both apply the slices
+// are faster from the smallest volumes on (one voxel, 16 -> 16: 8 against 15 us).
+constexpr size_t kSmemLimit = 227*1024, kSmemHalf = 113*1024, kSmemQuarter = 56*1024;
+
+bool planSlices(SliceParams& p, int sms, size_t& smem, int& grid) {
+    if (p.cin != 8 && p.cin%16 != 0)
+        return false;
+    p.colsX = (p.W + kTileX - 1)/kTileX;
+    p.colsY = (p.H + kTileY - 1)/kTileY;
+    const long long columns = (long long) p.colsX*p.colsY*p.batch;
+    if (columns*p.D > (1LL << 28) || (long long) p.H*p.W*p.cin >= (1LL << 31))
+        return false;
+    // Output channels per CTA: at most 112 (four accumulators in tensor memory), those with the least time by the MMAs
+    // alone, rounds of items times the cycles of an MMA (32 for up to 64 channels, its reading of A; then N/2): wide
+    // tiles read A less often, narrow ones spread few planes over more SMs.
+    long long best = -1;
+    for (int n = std::min(112, p.cout); n >= 16; n -= 16) {
+        if (p.cout%n != 0)
+            continue;
+        const long long cost = (columns*p.D*(p.cout/n) + sms - 1)/sms*std::max(32, n/2);
+        if (best < 0 || cost < best) {
+            best = cost;
+            p.nTile = n;
+        }
+    }
+    p.nBlocks = p.cout/p.nTile;
+    p.accSlots = p.nTile < 32 ? kMaxAcc : 4;
+    // Planes per item: long runs load fewer slices twice, short ones balance the SMs.
+    p.zLen = 8;
+    while (p.zLen > 1 && (columns*((p.D + p.zLen - 1)/p.zLen)*p.nBlocks < 3*sms || (p.cin == 8 && p.D%p.zLen != 0)))
+        p.zLen /= 2;
+    p.zBlocks = (p.D + p.zLen - 1)/p.zLen;
+    const long long items = columns*p.zBlocks*p.nBlocks;
+    p.items = (int) items;
+    // Slots, with all weights resident if they fit beside at least three slices (two CTAs per SM if those fit), else
+    // with a ring of weight tiles.  A CTA of several items keeps its weights only if all items have the same channels.
+    const bool keep = p.nBlocks == 1 || items <= sms;
+    auto fits = [&](int slots, int wSlots, size_t limit) {
+        if (sliceSmemBytes(p.cin, p.nTile, slots, wSlots) > limit)
+            return false;
+        p.slots = slots;
+        p.wSlots = wSlots;
+        return true;
+    };
+    bool found = false;
+    if (p.cin == 8) {
+        // The slots of an item are consecutive (a pair of taps spans two slices): two items' worth of them.
+        found = keep && fits(2*(p.zLen + 2), kTaps, kSmemLimit);
+    }
+    else {
+        for (size_t limit : {kSmemQuarter, kSmemHalf, kSmemLimit})
+            for (int slots = 6; slots >= 3 && keep && !found; slots--)
+                found = fits(slots, kTaps, limit);
+        for (int n = 8; n >= 4 && !found && items > sms; n--)
+            found = fits(3, n, kSmemHalf);
+        for (int n = 12; n >= 2 && !found; n--)
+            found = (p.zLen > 1 && fits(3, n, kSmemLimit)) || fits(2, n, kSmemLimit);
+    }
+    if (!found)
+        return false;
+    smem = sliceSmemBytes(p.cin, p.nTile, p.slots, p.wSlots);
+    // Several CTAs per SM where shared and tensor memory allow: one thread issues a CTA's MMAs and is slower than the
+    // tensor core on narrow layers.
+    int perSM = 1;
+    while (perSM < 4 && (smem + 1024)*(perSM + 1) <= kSmemLimit + 1024 && tmemColumns(p.accSlots*p.nTile)*(perSM + 1) <= 512)
+        perSM++;
+    grid = (int) std::min(items, (long long) perSM*sms);
+    return true;
+}
+
 LbmStatus launchError(cudaError_t e) {
     lbm::setLastError(std::string("conv3d: ") + cudaGetErrorString(e));
     return LBM_ERR_CUDA;
@@ -333,12 +878,34 @@ LbmStatus lbm_conv3d_forward(const void* x, const void* w, const float* bias, vo
     if (cin <= 0 || cin%8 != 0 || cout < 16 || cout > 256 || cout%16 != 0)
         return invalid("lbm_conv3d_forward: cin must be a multiple of 8 and cout a multiple of 16 up to 256");
     long long voxels = (long long) batch*depth*height*width;
-    size_t smem = stageBytes(cout);
-    cudaError_t e = cudaFuncSetAttribute(convForwardKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    SliceParams p;
+    p.x = (const __nv_bfloat16*) x;
+    p.w = (const __nv_bfloat16*) w;
+    p.bias = bias;
+    p.y = (__nv_bfloat16*) y;
+    p.batch = batch; p.D = depth; p.H = height; p.W = width; p.cin = cin; p.cout = cout; p.relu = relu;
+    int device = 0, sms = 148, grid = 0;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    size_t smem = 0;
+    cudaError_t e;
+    if (planSlices(p, sms, smem, grid)) {
+        const int mode = cin == 8 ? kSingleGroup : (p.wSlots == kTaps ? kResident : kStreamed);
+        auto kernel = mode == kSingleGroup ? convSliceKernel<kSingleGroup>
+                    : mode == kResident ? convSliceKernel<kResident> : convSliceKernel<kStreamed>;
+        const int threads = mode == kStreamed ? sliceThreads<kStreamed> : sliceThreads<kResident>;
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kSmemLimit);
+        if (e != cudaSuccess)
+            return launchError(e);
+        kernel<<<grid, threads, smem, (cudaStream_t) stream>>>(p);
+        e = cudaGetLastError();
+        return e == cudaSuccess ? LBM_OK : launchError(e);
+    }
+    smem = stageBytes(cout);
+    e = cudaFuncSetAttribute(convForwardKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
     if (e != cudaSuccess)
         return launchError(e);
-    unsigned grid = (unsigned) ((voxels + kTileM - 1)/kTileM);
-    convForwardKernel<<<grid, kThreads, smem, (cudaStream_t) stream>>>(
+    convForwardKernel<<<(unsigned) ((voxels + kTileM - 1)/kTileM), kThreads, smem, (cudaStream_t) stream>>>(
         (const __nv_bfloat16*) x, (const __nv_bfloat16*) w, bias, (__nv_bfloat16*) y, batch, depth, height, width, cin,
         cout, relu);
     e = cudaGetLastError();
