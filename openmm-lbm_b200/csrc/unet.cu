@@ -4,10 +4,10 @@
 //                       (zero padding), read in place from slices of x in shared memory
 //  convForwardKernel    the same for the channel counts that the slices do not serve: A gathered per 128 voxels, all
 //                       cout in one N tile (<= 256)
-//  convWeightGradKernel dW[cout][k] = sum_voxels dy[voxel][cout] A[voxel][k]; CTAs over (cout tile, k tile, voxel
-//                       split), the K dimension of the GEMM being the voxels; results added with FP32 atomics
+//  convSliceGradKernel  dW[cout][k] = sum_voxels dy[voxel][cout] A[voxel][k], the K dimension of the GEMMs being the
+//                       voxels, from slices of x and shifted copies of dy; results added with FP32 atomics
 //
-// The GEMM core of the gathering kernels: 128 x N tiles, K in stages of 64 BF16 (one 128-byte row).  All 128 threads gather a stage into
+// The GEMM core of the gathering kernel: 128 x N tiles, K in stages of 64 BF16 (one 128-byte row).  All 128 threads gather a stage into
 // shared memory in the canonical K-major layout with the 128-byte swizzle (8-row atoms of 128-byte rows, the 16-byte
 // chunk index XOR the row within the atom), make it visible to the tensor core's proxy, and one thread issues four
 // tcgen05.mma (K = 16 each, BF16 x BF16 -> FP32 in tensor memory) and commits them to an mbarrier that every
@@ -96,6 +96,16 @@ __device__ __forceinline__ void tmemLoad8(uint32_t addr, float v[8]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
     for (int i = 0; i < 8; i++)
         v[i] = __uint_as_float(r[i]);
+}
+
+// 16 consecutive FP32 accumulator columns of this thread's row (lane) from tensor memory.
+__device__ __forceinline__ void tmemLoad16(uint32_t addr, uint32_t (&v)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+                 "%14, %15}, [%16];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                   "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
+                   "=r"(v[15]) : "r"(addr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
 __host__ __device__ inline uint32_t tmemColumns(int n) {
@@ -604,12 +614,7 @@ convSliceKernel(const SliceParams p) {
                 __nv_bfloat16* out = p.y + ((((size_t) it.n*p.D + it.z0 + k)*p.H + yy)*p.W + xx)*p.cout + it.co0;
                 for (int col = 0; col < p.nTile; col += 16) {
                     uint32_t v[16];
-                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, "
-                                 "%13, %14, %15}, [%16];"
-                                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                                   "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
-                                   "=r"(v[15]) : "r"(d + (uint32_t) col));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    tmemLoad16(d + (uint32_t) col, v);
                     if (store) {
                         __align__(16) __nv_bfloat16 o[16];
 #pragma unroll
@@ -705,80 +710,293 @@ convForwardKernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __re
     releaseStage(st, ncols);
 }
 
-// dW[cout][k] += sum_m dy[m][cout] A[m][k]: A tile rows = cout (tile of 128), B tile rows = k (tile of nt), the GEMM's
-// K = voxels in stages of 64.  Both tiles are gathered transposed (voxel along the 128-byte rows).
-__global__ void __launch_bounds__(kThreads)
-convWeightGradKernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ dy, float* __restrict__ dw,
-                     int batch, int D, int H, int W, int cin, int cout, int nt) {
-    extern __shared__ uint8_t smemRaw[];
-    const uint32_t ncols = tmemColumns(nt);
-    Stage st = setupStage(smemRaw, nt, ncols);
-    const int tid = threadIdx.x, warp = tid/32, lane = tid%32;
-    const long long M = (long long) batch*D*H*W;
-    const int K = 27*cin;
-    const int co0 = blockIdx.x*kTileM, k0 = blockIdx.y*nt;
-    const long long stagesTotal = (M + kChunk - 1)/kChunk;
-    const uint32_t idesc = instrDescriptor(nt);
-    const int col = tid%kChunk, half = tid/kChunk;       // this thread's voxel column and row-group parity
-    const long long limit = convWaitPolls;
-    bool ok = true;
-    int stage = 0;
-    for (long long c = blockIdx.z; c < stagesTotal && ok; c += gridDim.z, stage++) {
-        const long long m = c*kChunk + col;
-        const bool valid = m < M;
-        int vx = 0, vy = 0, vz = 0, vn = 0;
-        if (valid) {
-            long long r = m;
-            vx = (int) (r%W); r /= W;
-            vy = (int) (r%H); r /= H;
-            vz = (int) (r%D); vn = (int) (r/D);
-        }
-        const uint32_t colOffset = (uint32_t) ((col & 7)*2);
-        // A: rows cout (16 groups of 8), column = this voxel.
-        for (int g = half; g < kTileM/8; g += 2) {
-            int co = co0 + 8*g;
-            uint4 val = make_uint4(0, 0, 0, 0);
-            if (valid && co < cout)
-                val = __ldg(reinterpret_cast<const uint4*>(dy + m*cout + co));
-            const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&val);
-            for (int i = 0; i < 8; i++)
-                *reinterpret_cast<__nv_bfloat16*>(st.tileA + swizzled(8*g + i, col >> 3) + colOffset) = e[i];
-        }
-        // B: rows k = k0 + 8 g + i (one tap and 8 channels per group), column = this voxel.
-        for (int g = half; g < nt/8; g += 2) {
-            int k = k0 + 8*g;
-            uint4 val = make_uint4(0, 0, 0, 0);
-            if (valid && k < K) {
-                int tap = k/cin, ci = k - tap*cin;
-                int zz = vz + tap/9 - 1, yy = vy + (tap/3)%3 - 1, xx = vx + tap%3 - 1;
-                if (zz >= 0 && zz < D && yy >= 0 && yy < H && xx >= 0 && xx < W)
-                    val = __ldg(reinterpret_cast<const uint4*>(x + ((((long long) vn*D + zz)*H + yy)*W + xx)*cin + ci));
-            }
-            const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&val);
-            for (int i = 0; i < 8; i++)
-                *reinterpret_cast<__nv_bfloat16*>(st.tileB + swizzled(8*g + i, col >> 3) + colOffset) = e[i];
-        }
-        ok = runStage(st, idesc, stage, limit);
-        if (!ok)
-            drainStage(st, stage);
+// ---------------------------------------------------------------------------------------------------------------
+// The weight gradient dw[co][tap][ci] += sum_v dy[v][co] x[v + tap][ci]: GEMMs whose K are the voxels, with both
+// operands in the unswizzled MN-major layout, 8 channels x 8 voxels of 16 bytes a core matrix, 16 x-neighbours (two
+// core matrices) per tcgen05.mma.  One MMA serves many taps at once:
+//   M (128 rows)  the channels of x on the rows y - 1, y, y + 1: [row][8-channel group] is one sequence of groups at
+//                 one stride, so 3 `groupsX` groups (at most 15 of the tile's 16) cover the taps' dy; what the other
+//                 rows of the tile read is never looked at
+//   N             the channels of dy in three copies, each shifted by one voxel in x: [dz][dx][8-channel group], again
+//                 at one stride: N = 3 coTile, or 9 coTile where all three planes fit into 256 columns
+// A CTA takes `groupsX` groups of input channels, coTile output channels and all dz (dzCount = 3), or one (more than 48
+// output channels: the accumulators of all would not fit into tensor memory).  It walks over its share of the items, columns
+// of 16 x 8 voxels (x, y) over zLen planes; warps 0-7 copy slices of x into a ring and the shifted copies of dy into two
+// buffers, warp 8 issues the MMAs, and warps 9-16 add finished sums to dw with FP32 atomics.
+//
+// The tensor core truncates its running sums: their relative error grows by about 2^-25 per MMA.  So a sum is handed to the
+// atomics (rounded to nearest) after `chain` MMAs at most, and the accumulators are a ring of units (all dz of an MMA, or
+// one) that are read and cleared while the next unit fills.
+//
+// Bound: 16 -> 16 channels read 4 KB of x and 4.6 KB of dy (68 wavefronts of shared memory) per MMA and 16 voxels, 19 us
+// on two 64 x 64 x 128 volumes.  Measured there: 90 us, what remains being the copies (dy three times) and the atomics of
+// the finished sums (65 us, with an error of 4e-6 instead of 9e-7, when a CTA adds its sums once); 1150 us with the
+// kernel before it, which gathered both operands transposed element by element and waited for each stage.  48 -> 16:
+// 180 us (4000), 32 -> 32 at 32 x 32 x 64 30 us (314), 160 -> 160 at 8 x 8 x 16 24 us (116).
+// ---------------------------------------------------------------------------------------------------------------
+
+constexpr int kRunX = 16, kRowsY = 8;
+constexpr int kGroupPitch = kRunX*16 + 16;     // bytes of a group's 16 voxels; + 16 spreads the groups over the banks
+constexpr int kGradSlots = 4;
+constexpr int kGradProducers = 256, kGradReaders = 256;
+constexpr int kGradThreads = kGradProducers + 32 + kGradReaders, kMaxUnits = 5;
+
+struct GradParams {
+    const __nv_bfloat16* x;
+    const __nv_bfloat16* dy;
+    float* dw;
+    int batch, D, H, W, cin, cout;
+    int groupsX, chunks, coTile, coBlocks, dzCount, zLen, chain;
+    int colsX, colsY, zBlocks, items;
+};
+
+struct GradBarriers {
+    uint64_t full[kGradSlots], empty[kGradSlots], dyEmpty[2], unitFull[kMaxUnits], unitEmpty[kMaxUnits], drain;
+    uint32_t tmem;
+    int stop;
+};
+
+__host__ __device__ inline int gradSliceBytes(int groupsX) { return (kRowsY + 2)*groupsX*kGroupPitch; }
+__host__ __device__ inline int gradDyBytes(int coTile, int zLen) { return kRowsY*zLen*3*(coTile/8)*kGroupPitch; }
+__host__ __device__ inline size_t gradSmemBytes(int groupsX, int coTile, int zLen) {
+    // The last row's tile reads 16 groups, 3 groupsX of which are its own.
+    return sizeof(GradBarriers) + 128 + (size_t) kGradSlots*gradSliceBytes(groupsX) + 16*kGroupPitch
+         + 2*(size_t) gradDyBytes(coTile, zLen);
+}
+
+__global__ void __launch_bounds__(kGradThreads)
+convSliceGradKernel(const GradParams p) {
+    extern __shared__ __align__(128) uint8_t smemRaw[];
+    GradBarriers* bars = reinterpret_cast<GradBarriers*>(smemRaw);
+    const int slotBytes = gradSliceBytes(p.groupsX), dyBytes = gradDyBytes(p.coTile, p.zLen);
+    const uint32_t ring = (smemAddr(smemRaw) + (uint32_t) sizeof(GradBarriers) + 127u) & ~127u;
+    const uint32_t dyBase = ring + (uint32_t) (kGradSlots*slotBytes + 16*kGroupPitch);
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid/32, 0), lane = tid%32;
+    const int width = 3*p.coTile;                     // columns per dz
+    // Accumulators: units of all dz (one MMA serves them) or of one.
+    const bool merged = p.dzCount*width <= 256;
+    const int unitsPerSum = merged ? 1 : p.dzCount, unitWidth = merged ? p.dzCount*width : width;
+    const int units = min(kMaxUnits, 512/unitWidth);
+    const uint32_t ncols = tmemColumns(units*unitWidth);
+    volatile int* stop = &bars->stop;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smemAddr(&bars->tmem)), "r"(ncols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    if (tid == 32) {
+        auto init = [](uint64_t* b, int count) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smemAddr(b)), "r"(count) : "memory");
+        };
+        for (int i = 0; i < kGradSlots; i++) {
+            init(&bars->full[i], kGradProducers);
+            init(&bars->empty[i], 1);
+        }
+        init(&bars->dyEmpty[0], 1);
+        init(&bars->dyEmpty[1], 1);
+        for (int i = 0; i < units; i++) {
+            init(&bars->unitFull[i], 1);
+            init(&bars->unitEmpty[i], kGradReaders);
+        }
+        init(&bars->drain, 1);
+        bars->stop = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    fenceBeforeSync();
+    __syncthreads();
     fenceAfterSync();
-    if (ok && stage > 0) {
-        const int row = warp*32 + lane, co = co0 + row;
-        for (int c0 = 0; c0 < nt; c0 += 8) {
-            float v[8];
-            tmemLoad8(st.tmem + ((uint32_t) (warp*32) << 16) + (uint32_t) c0, v);
-            if (co < cout)
-                for (int i = 0; i < 8; i++) {
-                    int k = k0 + c0 + i;
-                    if (k < K)
-                        atomicAdd(&dw[(long long) co*K + k], v[i]);
+    const uint32_t tmem = __shfl_sync(0xffffffffu, bars->tmem, 0);
+    // The accumulators start at zero, so that every MMA adds.  Warps 9-16 own the lanes 32 (warp % 4) and on, every other
+    // 16 columns each.
+    const uint32_t laneBase = tmem + ((uint32_t) (warp%4*32) << 16);
+    const int share = warp > kGradProducers/32 + 4 ? 16 : 0;
+    auto clear = [&](int from, int count) {
+        for (int c = from + share; c < from + count; c += 32)
+            for (int h = 0; h < 16; h += 8)
+                asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1};"
+                             :: "r"(laneBase + (uint32_t) (c + h)), "r"(0) : "memory");
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    };
+    if (warp > kGradProducers/32)
+        clear(0, units*unitWidth);
+    fenceBeforeSync();
+    __syncthreads();
+    fenceAfterSync();
+    const long long limit = convWaitPolls;
+    int block = blockIdx.y;
+    const int chunk = block%p.chunks; block /= p.chunks;
+    const int co0 = block%p.coBlocks*p.coTile;
+    const int dzOnly = p.dzCount == 3 ? 0 : block/p.coBlocks;
+    const int group0 = chunk*p.groupsX, groupsX = min(p.groupsX, p.cin/8 - group0), groupsY = p.coTile/8;
+    // Slices of an item: every plane's three with all dz, else the one that its dz reads.
+    const int halo = p.dzCount - 1;
+    auto item = [&](int i, int& n, int& z0, int& zc, int& y0, int& x0) {
+        x0 = i%p.colsX*kRunX; i /= p.colsX;
+        y0 = i%p.colsY*kRowsY; i /= p.colsY;
+        z0 = i%p.zBlocks*p.zLen;
+        n = i/p.zBlocks;
+        zc = min(p.zLen, p.D - z0);
+    };
+
+    if (warp < kGradProducers/32) {
+        CopyQueue queue;
+        const Pieces byX(tid, kGradProducers, groupsX), byY(tid, kGradProducers, groupsY);
+        int slot = 0, buffer = 0;
+        uint32_t slotPhase = 1, dyPhase = 1;         // a free slot's barrier has completed the phase before its first
+        bool ok = true;
+        for (int i = blockIdx.x; i < p.items && ok; i += gridDim.x) {
+            int n, z0, zc, y0, x0;
+            item(i, n, z0, zc, y0, x0);
+            ok = queue.waitFree(smemAddr(&bars->dyEmpty[buffer]), dyPhase, limit, stop);
+            for (int j = 0; j < zc + halo && ok; j++) {
+                if (j < zc) {
+                    // Plane z0 + j of dy: copy dx holds dy at x - (dx - 1).
+                    const __nv_bfloat16* plane = p.dy + ((size_t) n*p.D + z0 + j)*p.H*p.W*p.cout + co0;
+                    const uint32_t base = dyBase + (uint32_t) (buffer*dyBytes);
+                    for (int g = byY.g, v = byY.v; v < kRowsY*3*kRunX; ) {
+                        const int k = v%kRunX, r = v/kRunX, y = r/3, dx = r%3;
+                        const int yy = y0 + y, xx = x0 + k + 1 - dx;
+                        const bool valid = yy < p.H && (unsigned) xx < (unsigned) p.W;
+                        copy16(base + (uint32_t) ((((y*p.zLen + j)*3 + dx)*groupsY + g)*kGroupPitch + k*16),
+                               plane + (valid ? ((size_t) yy*p.W + xx)*p.cout + 8*g : 0), valid);
+                        byY.next(g, v);
+                    }
                 }
+                ok = queue.waitFree(smemAddr(&bars->empty[slot]), slotPhase, limit, stop);
+                if (!ok)
+                    break;
+                const int z = p.dzCount == 3 ? z0 + j - 1 : z0 + j + dzOnly - 1;
+                const bool inside = z >= 0 && z < p.D;
+                const __nv_bfloat16* plane = p.x + ((size_t) n*p.D + (inside ? z : 0))*p.H*p.W*p.cin + 8*group0;
+                const uint32_t base = ring + (uint32_t) (slot*slotBytes);
+                for (int g = byX.g, v = byX.v; v < (kRowsY + 2)*kRunX; ) {
+                    const int k = v%kRunX, y = v/kRunX, yy = y0 + y - 1, xx = x0 + k;
+                    const bool valid = inside && (unsigned) yy < (unsigned) p.H && xx < p.W;
+                    copy16(base + (uint32_t) ((y*groupsX + g)*kGroupPitch + k*16),
+                           plane + (valid ? ((size_t) yy*p.W + xx)*p.cin + 8*g : 0), valid);
+                    byX.next(g, v);
+                }
+                queue.push(smemAddr(&bars->full[slot]));
+                if (++slot == kGradSlots) {
+                    slot = 0;
+                    slotPhase ^= 1;
+                }
+            }
+            buffer ^= 1;
+            dyPhase ^= buffer == 0 ? 1 : 0;
+        }
+        queue.flush();
+    }
+    else if (warp == kGradProducers/32) {
+        // Both operands MN-major (bits 15 and 16 of the instruction descriptor).
+        const uint32_t high = (kGroupPitch >> 4) | (1u << 14), low = (128u >> 4) << 16;
+        const uint32_t rowX = (uint32_t) (groupsX*kGroupPitch) >> 4;
+        const uint32_t planeY = (uint32_t) (3*groupsY*kGroupPitch) >> 4, rowY = planeY*(uint32_t) p.zLen;
+        int slot = 0, buffer = 0, unit = 0, chain = 0;
+        uint32_t slotPhase = 0, unitPhase = 1;       // of the sum's first unit
+        bool ok = true, issued = false;
+        for (int i = blockIdx.x; i < p.items && ok; i += gridDim.x) {
+            int n, z0, zc, y0, x0;
+            item(i, n, z0, zc, y0, x0);
+            const int rows = min(kRowsY, p.H - y0);
+            // A new sum waits for its units to have been read and cleared.
+            for (int k = 0; k < unitsPerSum && ok && chain == 0; k++) {
+                const int at = unit + k;
+                ok = warpWait(smemAddr(&bars->unitEmpty[at%units]), unitPhase ^ (at >= units ? 1u : 0u), limit, stop);
+                fenceAfterSync();
+            }
+            for (int j = 0; j < zc + halo && ok; j++) {
+                ok = warpWait(smemAddr(&bars->full[slot]), slotPhase, limit, stop);
+                if (!ok)
+                    break;
+                // Slice j meets the planes k of dy with dz = j - k (all dz), in columns of their own, dz = 2 first.
+                const int first = max(0, j - halo), last = min(zc - 1, j);
+                const int count = last - first + 1, step = merged ? count : 1;
+                const uint32_t idesc = instrDescriptor(step*width) | (1u << 15) | (1u << 16);
+                uint32_t a = low | ((ring + (uint32_t) (slot*slotBytes)) >> 4);
+                uint32_t b = low | (((dyBase + (uint32_t) (buffer*dyBytes)) >> 4) + (uint32_t) first*planeY);
+                for (int y = 0; y < rows; y++, a += rowX, b += rowY)
+                    for (int k = 0; k < count; k += step) {
+                        const int column = halo - j + first + k, at = unit + column;
+                        mmaElected(tmem + (uint32_t) (merged ? unit*unitWidth + column*width : (at >= units ? at - units : at)*width),
+                                   join(a, high), join(b + (uint32_t) k*planeY, high), idesc, 1u);
+                    }
+                issued = true;
+                commitElected(smemAddr(&bars->empty[slot]));
+                if (++slot == kGradSlots) {
+                    slot = 0;
+                    slotPhase ^= 1;
+                }
+            }
+            if (!ok)
+                break;
+            commitElected(smemAddr(&bars->dyEmpty[buffer]));
+            buffer ^= 1;
+            chain += rows*zc;
+            if (chain + kRowsY > p.chain || i + (int) gridDim.x >= p.items) {
+                for (int k = 0; k < unitsPerSum; k++)
+                    commitElected(smemAddr(&bars->unitFull[(unit + k)%units]));
+                unit += unitsPerSum;
+                if (unit >= units) {
+                    unit -= units;
+                    unitPhase ^= 1;
+                }
+                chain = 0;
+            }
+        }
+        // The MMAs and arrivals in flight end before the CTA leaves.
+        if (issued) {
+            commitElected(smemAddr(&bars->drain));
+            waitParity(smemAddr(&bars->drain), 0, kSpinLimit);
+            __syncwarp();
         }
     }
-    else if (!ok && tid == 0)
+    else {
+        // Row 32 (warp % 4) + lane is (dy tap, channel group, channel), column ((2 - dz) 3 + dx) coTile + co.
+        const int row = warp%4*32 + lane, group = row/8;
+        const int ty = group/groupsX, ci = 8*(group0 + group%groupsX) + row%8;
+        int unit = 0, chain = 0;
+        uint32_t unitPhase = 0;
+        bool ok = true;
+        for (int i = blockIdx.x; i < p.items && ok; i += gridDim.x) {
+            int n, z0, zc, y0, x0;
+            item(i, n, z0, zc, y0, x0);
+            chain += min(kRowsY, p.H - y0)*zc;
+            if (chain + kRowsY <= p.chain && i + (int) gridDim.x < p.items)
+                continue;
+            chain = 0;
+            for (int k = 0; k < unitsPerSum && ok; k++) {
+                ok = warpWait(smemAddr(&bars->unitFull[unit]), unitPhase, limit, stop);
+                if (!ok)
+                    break;
+                fenceAfterSync();
+                for (int c = share; c < unitWidth; c += 32) {
+                    uint32_t v[16];
+                    tmemLoad16(laneBase + (uint32_t) (unit*unitWidth + c), v);
+                    const int co = c%p.coTile, r = c/p.coTile + 3*k, dx = r%3, dz = p.dzCount == 3 ? 2 - r/3 : dzOnly;
+                    if (ty < 3) {
+                        float* out = p.dw + ((size_t) (co0 + co)*kTaps + 9*dz + 3*ty + dx)*p.cin + ci;
+#pragma unroll
+                        for (int q = 0; q < 16; q++)
+                            atomicAdd(out + (size_t) q*kTaps*p.cin, __uint_as_float(v[q]));
+                    }
+                    __syncwarp();
+                }
+                clear(unit*unitWidth, unitWidth);
+                fenceBeforeSync();
+                arrive(smemAddr(&bars->unitEmpty[unit]));
+                if (++unit == units) {
+                    unit = 0;
+                    unitPhase ^= 1;
+                }
+            }
+        }
+    }
+    fenceBeforeSync();
+    __syncthreads();
+    if (tid == 0 && bars->stop)
         atomicExch(&convStatus, (int) LBM_ERR_DEVICE_TIMEOUT);
-    releaseStage(st, ncols);
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(ncols) : "memory");
 }
 
 size_t stageBytes(int rowsB) {
@@ -857,6 +1075,38 @@ bool planSlices(SliceParams& p, int sms, size_t& smem, int& grid) {
     return true;
 }
 
+// The division of a weight gradient; returns the shared memory of a CTA.
+size_t planGradient(GradParams& p, int sms, dim3& grid) {
+    // At most 15 of an M tile's 16 groups are used (three rows of up to 5 channel groups).
+    const int groups = p.cin/8;
+    p.chunks = (groups + 4)/5;
+    p.groupsX = (groups + p.chunks - 1)/p.chunks;
+    p.chunks = (groups + p.groupsX - 1)/p.groupsX;
+    // All dz of up to 48 output channels in one CTA (432 columns of tensor memory), else one dz of up to 80 (N <= 240).
+    auto divisor = [&](int most) {
+        int n = std::min(most, p.cout);
+        while (p.cout%n != 0)
+            n -= 16;
+        return n;
+    };
+    p.dzCount = p.cout <= 48 ? 3 : 1;
+    p.coTile = divisor(p.dzCount == 3 ? 48 : 80);
+    p.coBlocks = p.cout/p.coTile;
+    // MMAs per sum: an error of about 1e-6 on large volumes; small ones, whose sums are short anyway, keep theirs at 1e-7.
+    const long long runs = ((long long) p.W*p.H*p.D*p.batch + 15)/16, parts = ((p.cout + 127)/128)*(((long long) 27*p.cin + 255)/256);
+    p.chain = (int) std::max(8LL, std::min(p.dzCount == 3 ? 32LL : 48LL, runs/(4*sms/parts + 1)));
+    // Planes per item: as many as keep a buffer of dy within 75 KB (a slice of x is read by up to three planes).
+    p.zLen = p.dzCount == 3 ? std::max(1, std::min(4, 76800/gradDyBytes(p.coTile, 1))) : 1;
+    p.colsX = (p.W + kRunX - 1)/kRunX;
+    p.colsY = (p.H + kRowsY - 1)/kRowsY;
+    p.zBlocks = (p.D + p.zLen - 1)/p.zLen;
+    p.items = (int) ((long long) p.colsX*p.colsY*p.zBlocks*p.batch);
+    const size_t smem = gradSmemBytes(p.groupsX, p.coTile, p.zLen);
+    const int blocks = p.chunks*p.coBlocks*(p.dzCount == 3 ? 1 : 3);
+    grid = dim3((unsigned) std::max(1, std::min(p.items, sms/blocks)), (unsigned) blocks);
+    return smem;
+}
+
 LbmStatus launchError(cudaError_t e) {
     lbm::setLastError(std::string("conv3d: ") + cudaGetErrorString(e));
     return LBM_ERR_CUDA;
@@ -918,23 +1168,20 @@ LbmStatus lbm_conv3d_weight_grad(const void* x, const void* dy, float* dw, int b
         return invalid("lbm_conv3d_weight_grad: null pointer or empty volume");
     if (cin <= 0 || cin%8 != 0 || cout < 16 || cout > 256 || cout%16 != 0)
         return invalid("lbm_conv3d_weight_grad: cin must be a multiple of 8 and cout a multiple of 16 up to 256");
-    long long voxels = (long long) batch*depth*height*width;
-    int K = 27*cin;
-    int nt = ((K + 15)/16)*16;
-    if (nt > 256)
-        nt = 256;
+    GradParams p;
+    p.x = (const __nv_bfloat16*) x;
+    p.dy = (const __nv_bfloat16*) dy;
+    p.dw = dw;
+    p.batch = batch; p.D = depth; p.H = height; p.W = width; p.cin = cin; p.cout = cout;
     int device = 0, sms = 148;
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    unsigned gx = (unsigned) ((cout + kTileM - 1)/kTileM), gy = (unsigned) ((K + nt - 1)/nt);
-    long long stages = (voxels + kChunk - 1)/kChunk;
-    long long gz = std::max(1LL, std::min(stages, (long long) (4*sms)/(long long) (gx*gy) + 1));
-    size_t smem = stageBytes(nt);
-    cudaError_t e = cudaFuncSetAttribute(convWeightGradKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem);
+    dim3 grid;
+    const size_t smem = planGradient(p, sms, grid);
+    cudaError_t e = cudaFuncSetAttribute(convSliceGradKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) kSmemLimit);
     if (e != cudaSuccess)
         return launchError(e);
-    convWeightGradKernel<<<dim3(gx, gy, (unsigned) gz), kThreads, smem, (cudaStream_t) stream>>>(
-        (const __nv_bfloat16*) x, (const __nv_bfloat16*) dy, dw, batch, depth, height, width, cin, cout, nt);
+    convSliceGradKernel<<<grid, kGradThreads, smem, (cudaStream_t) stream>>>(p);
     e = cudaGetLastError();
     return e == cudaSuccess ? LBM_OK : launchError(e);
 }

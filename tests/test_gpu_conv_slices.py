@@ -36,3 +36,19 @@ def test_forward_at_the_edges_of_its_tiles(n, shape, cin, cout):
     ref = conv_oracle.conv3d_forward(x, w, b, False)
     got = y.float().permute(0, 2, 3, 4, 1).cpu().numpy()
     assert abs(got - ref).max() <= 2.0**-8*abs(ref).max()
+
+
+@pytest.mark.parametrize('n,shape,cin,cout', [
+    (1, (1, 1, 1), 16, 16), (1, (4, 8, 16), 8, 16), (2, (5, 9, 17), 16, 32), (1, (3, 7, 15), 48, 48),
+    (1, (9, 17, 33), 40, 16), (1, (3, 9, 18), 88, 64), (1, (2, 5, 20), 224, 160), (1, (4, 3, 5), 24, 112),
+    (1, (21, 40, 35), 16, 16)])
+def test_weight_gradient_at_the_edges_of_its_tiles(n, shape, cin, cout):
+    """FP32 sums of exact products, cut every 48 MMAs of 16 voxels at most: 48 truncations of 2^-24 and the atomics'
+    rounding, below 1e-5 of the largest entry."""
+    rng = np.random.default_rng(5*cin + cout + shape[2])
+    x = rounded(rng.standard_normal((n,) + shape + (cin,)))
+    dy = rounded(rng.standard_normal((n,) + shape + (cout,)))
+    g = ws.conv3d_weight_grad(volume(x), volume(dy))
+    ws.conv_status()
+    ref = conv_oracle.conv3d_weight_grad(x, dy)
+    assert abs(g.cpu().numpy() - ref).max() <= 1e-5*abs(ref).max()
