@@ -44,7 +44,8 @@ struct FluidView {
     const uint32_t* solidMask; // bit per node, rows padded to 32 bits; NULL without solid nodes
     const uint32_t* reactMask; // bit per node with a coupling reaction; NULL without particles
     const void* reaction;      // 4 values (R) per node, lattice units
-    double* partials;          // 4 doubles per block of the dense kernels
+    double* partials;          // a record per block of the step's passes
+    unsigned* ticket;          // blocks of the dense kernel that have stored their record (finishStep)
     StepStats* stats;          // statistics of the last step (ucm read by the next removal)
 };
 
