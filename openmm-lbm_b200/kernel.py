@@ -111,6 +111,9 @@ class B200Kernel:
         if hasattr(density, 'data_ptr'):
             assert density.is_cuda and density.dtype.itemsize == 8 and density.is_contiguous()
             assert velocity.is_cuda and velocity.dtype.itemsize == 8 and velocity.is_contiguous()
+            # The kernel's stream does not wait for the stream that torch computes the fields on.
+            import torch
+            torch.cuda.current_stream(density.device).synchronize()
             check(self.lib.lbm_set_fluid_equilibrium(self.handle, density.data_ptr(), velocity.data_ptr(), MEMORY_DEVICE,
                                                      int(strain)), self.lib)
             return
