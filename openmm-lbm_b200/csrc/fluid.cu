@@ -903,30 +903,31 @@ __global__ void equilibriumKernel(T* A, T* B, FluidView v, const double* density
     }
 }
 
-// Density and velocity u = j/rho + g/2 of every node, zero at solid nodes (nodeFields,
-// ReferenceLBMKernels.cpp:1349-1368).
+// Density [N] and velocity [N][3], u = j/rho + g/2, of every node, zero at solid nodes (nodeFields,
+// ReferenceLBMKernels.cpp:1349-1368), in the layout of the caller's arrays.
 template <typename T, typename R>
-__global__ void fieldsKernel(const T* A, FluidView v, double* out, double densityScale, double velocityScale) {
+__global__ void fieldsKernel(const T* A, FluidView v, double* density, double* velocity, double densityScale,
+                             double velocityScale) {
     for (long long x = blockIdx.x*(long long) blockDim.x + threadIdx.x; x < v.n; x += (long long) gridDim.x*blockDim.x) {
-        Coords c = nodeCoords(x, v.nx, v.ny);
-        long long row = (long long) c.z*v.ny + c.y;
+        const Coords c = nodeCoords(x, v.nx, v.ny);
+        const long long row = (long long) c.z*v.ny + c.y;
         if (v.solidMask != nullptr && ((v.solidMask[row*v.wordsPerRow + c.x/32] >> (c.x%32)) & 1u)) {
-            for (int k = 0; k < 4; k++)
-                out[4*x + k] = 0;
+            density[x] = velocity[3*x] = velocity[3*x+1] = velocity[3*x+2] = 0;
             continue;
         }
         double r = 1.0, jx = 0, jy = 0, jz = 0;
-        for (int q = 0; q < 19; q++) {
-            double fq = (double) loadq<T, R>(A + (long long) q*v.n + shifted(v, c.x, c.y, c.z, -cxr(q), -cyr(q), -czr(q)), q);
+        staticFor<19>([&](auto qc) {
+            constexpr int q = decltype(qc)::value;
+            const double fq = (double) loadq<T, R>(A + (long long) q*v.n + shifted(v, c.x, c.y, c.z, -cxOf(q), -cyOf(q), -czOf(q)), q);
             r += fq;
-            jx += cxr(q)*fq;
-            jy += cyr(q)*fq;
-            jz += czr(q)*fq;
-        }
-        out[4*x] = r*densityScale;
-        out[4*x+1] = (jx*(1.0/r) + v.g[0]*0.5)*velocityScale;
-        out[4*x+2] = (jy*(1.0/r) + v.g[1]*0.5)*velocityScale;
-        out[4*x+3] = (jz*(1.0/r) + v.g[2]*0.5)*velocityScale;
+            jx += cxOf(q)*fq;
+            jy += cyOf(q)*fq;
+            jz += czOf(q)*fq;
+        });
+        density[x] = r*densityScale;
+        velocity[3*x] = (jx*(1.0/r) + v.g[0]*0.5)*velocityScale;
+        velocity[3*x+1] = (jy*(1.0/r) + v.g[1]*0.5)*velocityScale;
+        velocity[3*x+2] = (jz*(1.0/r) + v.g[2]*0.5)*velocityScale;
     }
 }
 
@@ -1105,8 +1106,8 @@ struct Launcher {
     static void scatter(void* A, void* B, int q, const FluidView& v, const double* in, int* changed, cudaStream_t s) {
         scatterKernel<T, R><<<1184, 256, 0, s>>>((T*) A, (T*) B, q, v, in, changed);
     }
-    static void fields(const void* A, const FluidView& v, double* out, double ds, double vs, cudaStream_t s) {
-        fieldsKernel<T, R><<<1184, 256, 0, s>>>((const T*) A, v, out, ds, vs);
+    static void fields(const void* A, const FluidView& v, double* rho, double* u, double ds, double vs, cudaStream_t s) {
+        fieldsKernel<T, R><<<1184, 256, 0, s>>>((const T*) A, v, rho, u, ds, vs);
     }
 };
 
@@ -1167,6 +1168,7 @@ FluidEngine::FluidEngine(const LbmLatticeParameters& l, int storage, const Geome
         CUDA_CHECK(cudaMalloc(&pop[1], bytes));
         int device = 0, sms = 0;
         CUDA_CHECK(cudaGetDevice(&device));
+        hostCopy = HostCopy::forDevice(device);
         CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
         int occupancy = 1;
         dispatchStorage(storage, [&](auto L) { occupancy = decltype(L)::occupancy(); });
@@ -1230,12 +1232,16 @@ FluidEngine::FluidEngine(const LbmLatticeParameters& l, int storage, const Geome
         CUDA_CHECK(cudaStreamSynchronize(stream));
     }
     catch (...) {
-        this->~FluidEngine();
+        release();
         throw;
     }
 }
 
 FluidEngine::~FluidEngine() {
+    release();
+}
+
+void FluidEngine::release() {
     cudaFree(pop[0]);
     cudaFree(pop[1]);
     cudaFree(solidMaskDev);
@@ -1426,9 +1432,18 @@ StepStats FluidEngine::readStats() {
 }
 
 void FluidEngine::getState(double* host) {
-    getStateByDirection([&](int q, const double* values) {
-        std::memcpy(host + (size_t) q*view.n, values, sizeof(double)*view.n);
-    });
+    if (stagingDev == nullptr)
+        CUDA_CHECK(cudaMalloc(&stagingDev, sizeof(double)*4*(size_t) view.n));
+    // Four planes at a time, straight into the caller's array.
+    for (int q0 = 0; q0 < 19; q0 += 4) {
+        const int count = std::min(4, 19 - q0);
+        for (int k = 0; k < count; k++)
+            dispatchStorage(storageType, [&](auto L) {
+                decltype(L)::gather(pop[cur], q0 + k, view, (double*) stagingDev + (size_t) k*view.n, stream);
+            });
+        CUDA_CHECK(cudaGetLastError());
+        hostCopy->download({{host + (size_t) q0*view.n, stagingDev, sizeof(double)*(size_t) count*view.n}}, stream);
+    }
 }
 
 void FluidEngine::getStateByDirection(const std::function<void(int, const double*)>& sink) {
@@ -1497,18 +1512,14 @@ void FluidEngine::setEquilibrium(const double* density, const double* velocity, 
 void FluidEngine::fields(double* density, double* velocity, double densityScale, double velocityScale) {
     if (stagingDev == nullptr)
         CUDA_CHECK(cudaMalloc(&stagingDev, sizeof(double)*4*(size_t) view.n));
+    double* rho = (double*) stagingDev;
+    double* u = rho + view.n;
     dispatchStorage(storageType, [&](auto L) {
-        decltype(L)::fields(pop[cur], view, (double*) stagingDev, densityScale, velocityScale, stream);
+        decltype(L)::fields(pop[cur], view, rho, u, densityScale, velocityScale, stream);
     });
     CUDA_CHECK(cudaGetLastError());
-    std::vector<double> all(4*(size_t) view.n);
-    CUDA_CHECK(cudaMemcpyAsync(all.data(), stagingDev, sizeof(double)*all.size(), cudaMemcpyDeviceToHost, stream));
-    CUDA_CHECK(cudaStreamSynchronize(stream));
-    for (long long x = 0; x < view.n; x++) {
-        density[x] = all[4*x];
-        for (int a = 0; a < 3; a++)
-            velocity[3*x+a] = all[4*x+1+a];
-    }
+    hostCopy->download({{density, rho, sizeof(double)*(size_t) view.n}, {velocity, u, 3*sizeof(double)*(size_t) view.n}},
+                       stream);
 }
 
 void FluidEngine::copyStateOut(void* host) {

@@ -11,6 +11,7 @@
 // geometry but a one-bit solid mask per node.
 #pragma once
 
+#include "host_copy.h"
 #include "lbm_internal.h"
 #include <cuda_runtime.h>
 #include <functional>
@@ -99,7 +100,7 @@ public:
     long long launches;
 private:
     void launchStreamCollide(long long stepIndex, bool remove, bool react);
-    void launchFinish(int numBlocks, int numExtra);
+    void release();            // gives back the device memory and events
     LbmLatticeParameters lattice;
     int storageType;
     size_t elementSize;
@@ -123,6 +124,7 @@ private:
     double* faceDev;           // face velocities/densities and the boundary stress weight
     double* residualPrevDev = nullptr;   // 3N velocities of the last residual call
     double faceHost[32];
+    std::shared_ptr<HostCopy> hostCopy;  // of the fields and the state
     StepStats statsHost;
     bool profiling;
     std::vector<cudaEvent_t> profileEvents;   // start/stop pairs

@@ -1,0 +1,48 @@
+// Copies of large device arrays into the caller's (pageable) host memory.
+//
+// cudaMemcpy into pageable memory stages through the driver's buffers on one thread, which also takes the page faults of
+// a freshly allocated destination: 226 MB of fields (192^3) took 145 ms with the conversion around it.  Here several
+// threads each copy chunks through two pinned buffers of their own on a stream of their own, so that the transfer, the
+// copy into place and the page faults overlap: 15 ms.
+#pragma once
+
+#include "lbm_internal.h"
+#include <cuda_runtime.h>
+#include <memory>
+#include <mutex>
+#include <vector>
+
+namespace lbm {
+
+class HostCopy {
+public:
+    struct Piece {
+        void* host;
+        const void* device;
+        size_t bytes;
+    };
+    explicit HostCopy(int device) : device(device) {}
+    ~HostCopy();
+    // The copier of a device, shared by the kernels on it (pinned memory takes milliseconds to get): at most 8 MB of
+    // pinned memory, given back with the last kernel that holds it.
+    static std::shared_ptr<HostCopy> forDevice(int device);
+    HostCopy(const HostCopy&) = delete;
+    HostCopy& operator=(const HostCopy&) = delete;
+    // Copies the pieces once the work on `stream` is done; returns when they are in place.  One caller at a time: others
+    // wait for their turn (they would share the same link).
+    void download(const std::vector<Piece>& pieces, cudaStream_t stream);
+private:
+    struct Worker {
+        cudaStream_t stream = nullptr;
+        cudaEvent_t landed[2] = {nullptr, nullptr};
+    };
+    void prepare(int threads);
+    const int device;
+    std::mutex busy;
+    std::vector<Worker> workers;
+    char* pinned = nullptr;        // two chunks per worker
+    int pinnedWorkers = 0;
+    cudaEvent_t ready = nullptr;
+};
+
+} // namespace lbm

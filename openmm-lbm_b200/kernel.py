@@ -87,8 +87,8 @@ class B200Kernel:
         check(self.lib.lbm_copy_parameters(self.handle, ctypes.byref(self.lattice)), self.lib)
 
     def get_fluid_fields(self):
-        density = np.zeros(self.num_nodes)
-        velocity = np.zeros((self.num_nodes, 3))
+        density = np.empty(self.num_nodes)
+        velocity = np.empty((self.num_nodes, 3))
         check(self.lib.lbm_get_fluid_fields(self.handle, dptr(density), dptr(velocity)), self.lib)
         return density, velocity
 
@@ -151,7 +151,7 @@ class B200Kernel:
         return force
 
     def get_fluid_state(self):
-        state = np.zeros(19*self.num_nodes)
+        state = np.empty(19*self.num_nodes)
         check(self.lib.lbm_get_fluid_state(self.handle, dptr(state)), self.lib)
         return state
 
