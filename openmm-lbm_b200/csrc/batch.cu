@@ -1,8 +1,8 @@
 // Replica batches (include/lbm_b200_batch.h): independent periodic lattices of uneven sizes, each with its own beads,
 // advanced together.  Every phase of a step is one persistent launch over all replicas:
 //
-//  batchPairKernel            bead pair forces, one block per replica, all pairs (WCA / truncated Lennard-Jones)
-//  batchStencilKernel         stencil slots of every bead (node, weight, pulled fluid velocity), one thread per slot
+//  batchPairKernel            bead pair forces, one warp per bead, all pairs (WCA / truncated Lennard-Jones)
+//  batchStencilKernel         stencil slots of every bead (node, weight, pulled fluid velocity), one warp per bead
 //  batchExplicitKernel        explicit drag of every bead and its reaction on the fluid, one warp per bead
 //  batchStreamCollideKernel   the dense step of every replica: work items of BT consecutive nodes of one replica,
 //                             the node body of the single-lattice kernel (collide.cuh), per-warp partial sums
@@ -272,19 +272,19 @@ batchFinishKernel(const double* __restrict__ partials, const ReplicaTable* __res
 template <typename T, typename R>
 __global__ void __launch_bounds__(kBatchThreads)
 batchStencilKernel(const T* __restrict__ A, const FluidView* __restrict__ views, const CouplingView* __restrict__ cviews,
-                   const ReplicaTable* __restrict__ table, const int* __restrict__ particleReplica, long long totalSlots,
+                   const ReplicaTable* __restrict__ table, const int* __restrict__ particleReplica, int totalParticles,
                    int slots, const double* __restrict__ pos, const BatchClock* clock, int* slotNode, R* slotWeight,
                    typename Vec4<R>::type* slotU) {
     const long long step = clock->step;
-    for (long long t = blockIdx.x*(long long) blockDim.x + threadIdx.x; t < totalSlots; t += (long long) gridDim.x*blockDim.x) {
-        int p = (int) (t/slots), s = (int) (t - (long long) p*slots);
-        int r = particleReplica[p];
+    const int lane = threadIdx.x & 31, warps = (gridDim.x*blockDim.x) >> 5;
+    for (int p = (blockIdx.x*blockDim.x + threadIdx.x) >> 5; p < totalParticles; p += warps) {
+        const int r = particleReplica[p];
         const ReplicaTable& rt = table[r];
-        int p0 = rt.firstParticle, i = p - p0;
-        int remove = rt.removeFrequency > 0 && step%rt.removeFrequency == 0;
-        size_t so = (size_t) p0*slots;
-        stencilSlot<T, R>(A + (size_t) 19*rt.nodeOffset, views[r], cviews[r], pos + 3*(size_t) p0,
-                          (long long) i*slots + s, remove, 0, slotNode + so, slotWeight + so, slotU + so);
+        const int p0 = rt.firstParticle;
+        const int remove = rt.removeFrequency > 0 && step%rt.removeFrequency == 0;
+        const size_t so = (size_t) p0*slots;
+        stencilParticle<T, R>(A + (size_t) 19*rt.nodeOffset, views[r], cviews[r], pos + 3*(size_t) p0, p - p0, lane, remove,
+                              slotNode + so, slotWeight + so, slotU + so);
     }
 }
 
@@ -325,40 +325,54 @@ batchClearKernel(const FluidView* __restrict__ views, const int* __restrict__ pa
     }
 }
 
-// Pair force on bead i of a replica from all others, minimum image (the pair force of the bead dynamics, md.cu).
-__global__ void __launch_bounds__(kBatchThreads)
-batchPairKernel(const ReplicaTable* __restrict__ table, int numReplicas, PairParams pp, const double* __restrict__ pos,
-                double* fpair) {
-    for (int r = blockIdx.x; r < numReplicas; r += gridDim.x) {
-        const ReplicaTable& rt = table[r];
-        const double* x = pos + 3*(size_t) rt.firstParticle;
-        double* out = fpair + 3*(size_t) rt.firstParticle;
-        for (int i = threadIdx.x; i < rt.numParticles; i += blockDim.x) {
-            double f[3] = {0, 0, 0};
-            if (pp.type != LBM_PAIR_NONE)
-                for (int j = 0; j < rt.numParticles; j++) {
-                    if (j == i)
-                        continue;
-                    double d[3];
-                    for (int a = 0; a < 3; a++) {
-                        d[a] = x[3*i+a] - x[3*j+a];
-                        d[a] -= rt.box[a]*rint(d[a]/rt.box[a]);
-                    }
-                    double r2 = d[0]*d[0] + d[1]*d[1] + d[2]*d[2];
-                    if (r2 >= pp.rc2 || r2 == 0.0)
-                        continue;
-                    double s2 = pp.sigma2/r2, s6 = s2*s2*s2;
-                    double scale = 24.0*pp.eps*s6*(2.0*s6 - 1.0)/r2;
-                    for (int a = 0; a < 3; a++)
-                        f[a] += scale*d[a];
-                }
+// Pair force on bead i of a replica from all others, minimum image (the pair force of the bead dynamics, md.cu), by one
+// warp, its lanes over the others.  COHERENT: the positions were written by the same launch.  A block per replica with a
+// thread per bead left most of the GPU idle for up to 200 others in turn, each with three divisions (75 us per step of 96
+// replicas and 10,530 beads).
+template <bool COHERENT>
+__device__ __forceinline__ void pairForce(const ReplicaTable& rt, const PairParams& pp, const double* pos, int p, int lane,
+                                          double* fpair) {
+    const double* x = pos + 3*(size_t) rt.firstParticle;
+    const int i = p - rt.firstParticle, n = rt.numParticles;
+    auto at = [&](int k) { return COHERENT ? __ldcg(x + k) : x[k]; };
+    double f[3] = {0, 0, 0};
+    if (pp.type != LBM_PAIR_NONE) {
+        const double xi[3] = {at(3*i), at(3*i+1), at(3*i+2)};
+#pragma unroll 2
+        for (int j = lane; j < n; j += 32) {
+            double d[3];
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                d[a] = xi[a] - at(3*j+a);
+                d[a] -= rt.box[a]*rint(d[a]/rt.box[a]);
+            }
+            const double r2 = d[0]*d[0] + d[1]*d[1] + d[2]*d[2];
+            if (j == i || r2 >= pp.rc2 || r2 == 0.0)
+                continue;
+            const double s2 = pp.sigma2/r2, s6 = s2*s2*s2;
+            const double scale = 24.0*pp.eps*s6*(2.0*s6 - 1.0)/r2;
+#pragma unroll
             for (int a = 0; a < 3; a++)
-                out[3*i+a] = f[a];
+                f[a] += scale*d[a];
         }
     }
+    __syncwarp();
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+        f[a] = warpReduceSum(f[a]);
+    if (lane == 0)
+        for (int a = 0; a < 3; a++)
+            fpair[3*(size_t) p + a] = f[a];
 }
 
-// Leapfrog of every bead with the bead forces plus the drag: v += dt F/m, x += dt v (the bead dynamics' integrator).
+__global__ void __launch_bounds__(kBatchThreads)
+batchPairKernel(const ReplicaTable* __restrict__ table, const int* __restrict__ particleReplica, int totalParticles,
+                PairParams pp, const double* __restrict__ pos, double* fpair) {
+    const int lane = threadIdx.x & 31, warps = (gridDim.x*blockDim.x) >> 5;
+    for (int p = (blockIdx.x*blockDim.x + threadIdx.x) >> 5; p < totalParticles; p += warps)
+        pairForce<false>(table[particleReplica[p]], pp, pos, p, lane, fpair);
+}
+
 __global__ void __launch_bounds__(kBatchThreads)
 batchLeapfrogKernel(const ReplicaTable* __restrict__ table, const int* __restrict__ particleReplica, int totalParticles,
                     const double* __restrict__ invMass, const double* __restrict__ fpair, const double* __restrict__ fdrag,
@@ -374,50 +388,76 @@ batchLeapfrogKernel(const ReplicaTable* __restrict__ table, const int* __restric
     }
 }
 
-// Fluid and bead temperatures of every replica (one block each).
+// Sums of the temperatures over a chunk of kTemperatureNodes nodes of a replica (block x of replica y): rho, rho u and
+// (rho u)^2/rho with u = j/rho + g/2, per chunk in `partials`.  One block per replica took 2.7 ms for 96 replicas of up to
+// 64^3 nodes (a thousand nodes in turn per thread, with 64-bit divisions).
+constexpr int kTemperatureNodes = 2048, kTemperatureSums = 5;
+
 template <typename T>
 __global__ void __launch_bounds__(kBatchThreads)
 batchTemperatureKernel(const T* __restrict__ pop, const FluidView* __restrict__ views, const ReplicaTable* __restrict__ table,
-                       int numReplicas, const double* cellEnergy, const double* __restrict__ vel,
-                       const double* __restrict__ masses, double* out) {
-    __shared__ double red[kBatchThreads/32][8];
+                       double* __restrict__ partials) {
+    __shared__ double red[kBatchThreads/32][kTemperatureSums];
     const int lane = threadIdx.x%32, warp = threadIdx.x/32;
-    for (int r = blockIdx.x; r < numReplicas; r += gridDim.x) {
-        const FluidView& f = views[r];
-        const ReplicaTable& rt = table[r];
-        const T* A = pop + (size_t) 19*rt.nodeOffset;
-        double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (unsigned node = threadIdx.x; node < rt.numNodes; node += blockDim.x) {
-            double dr, jx, jy, jz;
-            pullMoments<T>(A, f, node, dr, jx, jy, jz);
-            double rho = 1.0 + dr;
-            double p[3] = {jx + 0.5*rho*f.g[0], jy + 0.5*rho*f.g[1], jz + 0.5*rho*f.g[2]};
-            acc[0] += rho;
-            for (int a = 0; a < 3; a++) {
-                acc[1+a] += p[a];
-                acc[4] += p[a]*p[a]/rho;
-            }
+    const ReplicaTable& rt = table[blockIdx.y];
+    const unsigned first = blockIdx.x*kTemperatureNodes;
+    if (first >= rt.numNodes)
+        return;
+    const FluidView& f = views[blockIdx.y];
+    const T* A = pop + (size_t) 19*rt.nodeOffset;
+    double acc[kTemperatureSums] = {0, 0, 0, 0, 0};
+    const unsigned end = min(rt.numNodes, first + kTemperatureNodes);
+    for (unsigned node = first + threadIdx.x; node < end; node += blockDim.x) {
+        const unsigned row = node/(unsigned) f.nx;
+        double dr, jx, jy, jz;
+        pullMomentsAt<T>(A, f, (int) (node - row*(unsigned) f.nx), (int) (row%(unsigned) f.ny), (int) (row/(unsigned) f.ny),
+                         dr, jx, jy, jz);
+        const double rho = 1.0 + dr;
+        const double p[3] = {jx + 0.5*rho*f.g[0], jy + 0.5*rho*f.g[1], jz + 0.5*rho*f.g[2]};
+        acc[0] += rho;
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            acc[1+a] += p[a];
+            acc[4] += p[a]*p[a]/rho;
         }
-        for (int i = threadIdx.x; i < rt.numParticles; i += blockDim.x) {
-            const double* v = vel + 3*(size_t) (rt.firstParticle + i);
-            acc[5] += masses[rt.firstParticle + i]*(v[0]*v[0] + v[1]*v[1] + v[2]*v[2]);
-        }
-        for (int k = 0; k < 6; k++)
-            acc[k] = warpReduceSum(acc[k]);
-        if (lane == 0)
-            for (int k = 0; k < 6; k++)
-                red[warp][k] = acc[k];
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double t[6] = {0, 0, 0, 0, 0, 0};
-            for (int w = 0; w < (int) blockDim.x/32; w++)
-                for (int k = 0; k < 6; k++)
-                    t[k] += red[w][k];
-            double mean2 = (t[1]*t[1] + t[2]*t[2] + t[3]*t[3])/t[0];
-            out[2*r] = (t[4] - mean2)/(3.0*rt.numNodes)*cellEnergy[r];
-            out[2*r+1] = rt.numParticles > 0 ? t[5]/(3.0*rt.numParticles) : 0.0;
-        }
-        __syncthreads();
+    }
+#pragma unroll
+    for (int k = 0; k < kTemperatureSums; k++)
+        acc[k] = warpReduceSum(acc[k]);
+    if (lane == 0)
+        for (int k = 0; k < kTemperatureSums; k++)
+            red[warp][k] = acc[k];
+    __syncthreads();
+    if (threadIdx.x < kTemperatureSums) {
+        double t = 0;
+        for (int w = 0; w < kBatchThreads/32; w++)
+            t += red[w][threadIdx.x];
+        partials[((size_t) blockIdx.y*gridDim.x + blockIdx.x)*kTemperatureSums + threadIdx.x] = t;
+    }
+}
+
+// The temperatures of replica blockIdx.x from its chunks' sums and its beads, by one warp.
+__global__ void __launch_bounds__(32)
+batchTemperatureSumKernel(const ReplicaTable* __restrict__ table, const double* __restrict__ partials, int chunks,
+                          const double* cellEnergy, const double* __restrict__ vel, const double* __restrict__ masses,
+                          double* out) {
+    const int r = blockIdx.x, lane = threadIdx.x;
+    const ReplicaTable& rt = table[r];
+    const int count = (int) ((rt.numNodes + kTemperatureNodes - 1)/kTemperatureNodes);
+    double t[kTemperatureSums + 1] = {0, 0, 0, 0, 0, 0};
+    for (int c = lane; c < count; c += 32)
+        for (int k = 0; k < kTemperatureSums; k++)
+            t[k] += partials[((size_t) r*chunks + c)*kTemperatureSums + k];
+    for (int i = lane; i < rt.numParticles; i += 32) {
+        const double* v = vel + 3*(size_t) (rt.firstParticle + i);
+        t[5] += masses[rt.firstParticle + i]*(v[0]*v[0] + v[1]*v[1] + v[2]*v[2]);
+    }
+    for (int k = 0; k <= kTemperatureSums; k++)
+        t[k] = warpReduceSum(t[k]);
+    if (lane == 0) {
+        const double mean2 = (t[1]*t[1] + t[2]*t[2] + t[3]*t[3])/t[0];
+        out[2*r] = (t[4] - mean2)/(3.0*rt.numNodes)*cellEnergy[r];
+        out[2*r+1] = rt.numParticles > 0 ? t[5]/(3.0*rt.numParticles) : 0.0;
     }
 }
 
@@ -485,9 +525,16 @@ __device__ __forceinline__ void finishReplica(const PersistentArgs& a, int r, in
     const ReplicaTable& rt = a.table[r];
     size_t begin = (size_t) rt.firstItem*warpsPerItem, count = (size_t) rt.numItems*warpsPerItem;
     double acc[4] = {0, 0, 0, 0};
-    for (size_t i = threadIdx.x; i < count; i += blockDim.x)
-        for (int k = 0; k < 4; k++)
-            acc[k] += __ldcg(&a.partials[4*(begin + i) + k]);
+    // The largest replicas have thousands of records: several are in flight per thread.
+#pragma unroll 4
+    for (size_t i = threadIdx.x; i < count; i += blockDim.x) {
+        const double2* record = reinterpret_cast<const double2*>(a.partials + 4*(begin + i));
+        const double2 low = __ldcg(record), high = __ldcg(record + 1);
+        acc[0] += low.x;
+        acc[1] += low.y;
+        acc[2] += high.x;
+        acc[3] += high.y;
+    }
     for (int k = 0; k < 4; k++)
         acc[k] = warpReduceSum(acc[k]);
     if (lane == 0)
@@ -510,18 +557,13 @@ __device__ __forceinline__ void finishReplica(const PersistentArgs& a, int r, in
     __syncthreads();
 }
 
-constexpr int kPairTile = 256;     // beads per shared-memory tile of the pair forces
-
 template <typename T, typename R, bool FLUCT, int BT>
 __global__ void __launch_bounds__(BT, batchMinBlocks<R, BT>())
 batchPersistentKernel(PersistentArgs a) {
     typedef typename Vec4<R>::type V;
-    __shared__ double pairTile[3*kPairTile];
     const int lane = threadIdx.x%32, warp = threadIdx.x/32;
     const long long step0 = a.clock->step;
-    const long long totalSlots = (long long) a.totalParticles*a.slots;
-    const int threads = gridDim.x*blockDim.x, firstThread = blockIdx.x*blockDim.x + threadIdx.x;
-    const int warps = threads >> 5, firstWarp = firstThread >> 5;
+    const int warps = (gridDim.x*blockDim.x) >> 5, firstWarp = (blockIdx.x*blockDim.x + threadIdx.x) >> 5;
     R* slotWeight = (R*) a.slotWeight;
     V* slotU = (V*) a.slotU;
     for (int s = 0; s < a.steps; s++) {
@@ -535,70 +577,30 @@ batchPersistentKernel(PersistentArgs a) {
             for (int r = blockIdx.x; r < a.numReplicas; r += gridDim.x)
                 finishReplica(a, r, BT/32);
         if (a.coupled) {
-            // Pair forces, all pairs of each replica in bead order (as batchPairKernel).  The positions were written in
-            // this launch by other blocks: they are read once through L2 into shared-memory tiles, which every bead of
-            // the block then reads.
-            for (int r = blockIdx.x; r < a.numReplicas; r += gridDim.x) {
-                const ReplicaTable& rt = a.table[r];
-                const double* x = a.pos + 3*(size_t) rt.firstParticle;
-                double* out = a.fpair + 3*(size_t) rt.firstParticle;
-                const int n = rt.numParticles;
-                for (int i0 = 0; i0 < n; i0 += blockDim.x) {
-                    const int i = i0 + threadIdx.x;
-                    double xi[3] = {0, 0, 0}, f[3] = {0, 0, 0};
-                    if (i < n)
-                        for (int k = 0; k < 3; k++)
-                            xi[k] = __ldcg(&x[3*i+k]);
-                    for (int j0 = 0; j0 < n && a.pair.type != LBM_PAIR_NONE; j0 += kPairTile) {
-                        const int count = min(kPairTile, n - j0);
-                        __syncthreads();
-                        for (int e = threadIdx.x; e < 3*count; e += blockDim.x)
-                            pairTile[e] = __ldcg(&x[3*j0 + e]);
-                        __syncthreads();
-                        if (i >= n)
-                            continue;
-                        for (int jj = 0; jj < count; jj++) {
-                            if (j0 + jj == i)
-                                continue;
-                            double d[3];
-                            for (int k = 0; k < 3; k++) {
-                                d[k] = xi[k] - pairTile[3*jj+k];
-                                d[k] -= rt.box[k]*rint(d[k]/rt.box[k]);
-                            }
-                            double r2 = d[0]*d[0] + d[1]*d[1] + d[2]*d[2];
-                            if (r2 >= a.pair.rc2 || r2 == 0.0)
-                                continue;
-                            double s2 = a.pair.sigma2/r2, s6 = s2*s2*s2;
-                            double scale = 24.0*a.pair.eps*s6*(2.0*s6 - 1.0)/r2;
-                            for (int k = 0; k < 3; k++)
-                                f[k] += scale*d[k];
-                        }
-                    }
-                    if (i < n)
-                        for (int k = 0; k < 3; k++)
-                            out[3*i+k] = f[k];
-                }
-            }
+            // A warp per bead: its pair force, the clear of its slots of the previous step (reaction buffer 1 - buf), and
+            // its slots of this step with the nodes' j/rho before the removal (applied in phase 2).  The positions were
+            // written in this launch by other blocks.
             int* nodes = a.slotNode[buf];
             const int* oldNodes = a.slotNode[1 - buf];
             const FluidView* oldViews = a.views[1 - buf];
-            for (long long t = firstThread; t < totalSlots; t += threads) {
-                const int p = (int) (t/a.slots), sl = (int) (t - (long long) p*a.slots);
+            for (int p = firstWarp; p < a.totalParticles; p += warps) {
                 const int r = a.particleReplica[p];
                 const ReplicaTable& rt = a.table[r];
-                const int p0 = rt.firstParticle, i = p - p0;
+                const int p0 = rt.firstParticle;
                 const size_t so = (size_t) p0*a.slots;
-                // The clear of slot t of the previous step (reaction buffer 1 - buf).
                 const FluidView& of = oldViews[r];
-                const long long node = __ldcg(&oldNodes[t]);
-                R* reaction = (R*) const_cast<void*>(of.reaction);
-                *reinterpret_cast<V*>(reaction + 4*node) = Vec4<R>::make(0, 0, 0, 0);
-                const long long row = node/of.nx;
-                const int xx = (int) (node - row*of.nx);
-                const_cast<uint32_t*>(of.reactMask)[row*of.wordsPerRow + xx/32] = 0u;
-                // The slot with the nodes' j/rho before the removal (applied in phase 2).
-                stencilSlot<T, R, true>(A + (size_t) 19*rt.nodeOffset, views[r], a.cviews[r], a.pos + 3*(size_t) p0,
-                                        (long long) i*a.slots + sl, 0, 0, nodes + so, slotWeight + so, slotU + so);
+                for (int s = lane; s < a.slots; s += 32) {
+                    const unsigned node = (unsigned) __ldcg(&oldNodes[(size_t) p*a.slots + s]);
+                    R* reaction = (R*) const_cast<void*>(of.reaction);
+                    *reinterpret_cast<V*>(reaction + 4*(size_t) node) = Vec4<R>::make(0, 0, 0, 0);
+                    const unsigned row = node/(unsigned) of.nx;
+                    const int xx = (int) (node - row*(unsigned) of.nx);
+                    const_cast<uint32_t*>(of.reactMask)[(size_t) row*of.wordsPerRow + xx/32] = 0u;
+                }
+                stencilParticle<T, R, true>(A + (size_t) 19*rt.nodeOffset, views[r], a.cviews[r], a.pos + 3*(size_t) p0,
+                                            p - p0, lane, 0, nodes + so, slotWeight + so, slotU + so);
+                __syncwarp();
+                pairForce<true>(rt, a.pair, a.pos, p, lane, a.fpair);
             }
         }
         if (!gridSync(a.barrier, a.status, a.pollLimit))
@@ -751,6 +753,7 @@ private:
     BatchClock* clockDev;
     int* itemReplicaDev;
     double* partialsDev;
+    double* temperatureDev = nullptr;    // the temperatures and their chunks' sums
     void* reactionDev;
     uint32_t* maskDev;
     int* particleReplicaDev;
@@ -977,7 +980,7 @@ void BatchEngine::release() {
     if (stream)
         cudaStreamSynchronize(stream);
     releaseGraph();
-    void* ptrs[] = {pop[0], pop[1], viewsDev, cviewsDev, tableDev, statsDev, clockDev, itemReplicaDev, partialsDev,
+    void* ptrs[] = {temperatureDev, pop[0], pop[1], viewsDev, cviewsDev, tableDev, statsDev, clockDev, itemReplicaDev, partialsDev,
                     reactionDev, maskDev, particleReplicaDev, posDev, velDev, fpairDev, fdragDev, invMassDev, massDev,
                     cellMassDev, wallDev, cellEnergyDev, slotNodeDev, slotWeightDev, slotUDev, statusDev};
     for (void* p : ptrs)
@@ -1066,9 +1069,10 @@ void BatchEngine::launchStep() {
     const T* A = (const T*) pop[cur];
     T* B = (T*) pop[1 - cur];
     if (coupled) {
-        batchPairKernel<<<std::min(numReplicas, sms*8), kBatchThreads, 0, stream>>>(tableDev, numReplicas, pairParams, posDev, fpairDev);
-        batchStencilKernel<T, R><<<gridS, kBatchThreads, 0, stream>>>(A, viewsDev, cviewsDev, tableDev, particleReplicaDev,
-                                                                      totalSlots, slots, posDev, clockDev, slotNodeDev,
+        batchPairKernel<<<gridP, kBatchThreads, 0, stream>>>(tableDev, particleReplicaDev, totalParticles, pairParams, posDev,
+                                                             fpairDev);
+        batchStencilKernel<T, R><<<gridP, kBatchThreads, 0, stream>>>(A, viewsDev, cviewsDev, tableDev, particleReplicaDev,
+                                                                      totalParticles, slots, posDev, clockDev, slotNodeDev,
                                                                       (R*) slotWeightDev, (typename Vec4<R>::type*) slotUDev);
         batchExplicitKernel<R><<<gridP, kBatchThreads, 0, stream>>>(viewsDev, cviewsDev, tableDev, particleReplicaDev,
                                                                     totalParticles, slots, velDev, slotNodeDev,
@@ -1360,24 +1364,31 @@ void BatchEngine::getFluidState(int r, double* state) {
 void BatchEngine::temperatures(double* fluidKT, double* beadKT) {
     CUDA_CHECK(cudaSetDevice(device));
     checkStatus();
-    CUDA_CHECK(cudaSetDevice(device));
-    double* out = nullptr;
-    CUDA_CHECK(cudaMalloc(&out, sizeof(double)*2*numReplicas));
-    int grid = std::min(numReplicas, sms*8);
-    if (storage == LBM_STORAGE_F64)
-        batchTemperatureKernel<double><<<grid, kBatchThreads, 0, stream>>>((const double*) pop[cur], viewsDev, tableDev,
-                                                                           numReplicas, cellEnergyDev, velDev, cellMassDev, out);
-    else
-        batchTemperatureKernel<float><<<grid, kBatchThreads, 0, stream>>>((const float*) pop[cur], viewsDev, tableDev,
-                                                                          numReplicas, cellEnergyDev, velDev, cellMassDev, out);
+    unsigned most = 1;
+    for (const ReplicaTable& t : tableHost)
+        most = std::max(most, t.numNodes);
+    const int chunks = (int) ((most + kTemperatureNodes - 1)/kTemperatureNodes);
+    if (temperatureDev == nullptr)
+        CUDA_CHECK(cudaMalloc(&temperatureDev, sizeof(double)*(2 + (size_t) chunks*kTemperatureSums)*numReplicas));
+    double* out = temperatureDev;
+    double* partials = temperatureDev + 2*(size_t) numReplicas;
+    // Replicas along y, in strips of at most 65,535.
+    for (int r0 = 0; r0 < numReplicas; r0 += 65535) {
+        const dim3 grid(chunks, std::min(65535, numReplicas - r0));
+        double* part = partials + (size_t) r0*chunks*kTemperatureSums;
+        if (storage == LBM_STORAGE_F64)
+            batchTemperatureKernel<double><<<grid, kBatchThreads, 0, stream>>>((const double*) pop[cur], viewsDev + r0,
+                                                                               tableDev + r0, part);
+        else
+            batchTemperatureKernel<float><<<grid, kBatchThreads, 0, stream>>>((const float*) pop[cur], viewsDev + r0,
+                                                                              tableDev + r0, part);
+        CUDA_CHECK(cudaGetLastError());
+    }
+    batchTemperatureSumKernel<<<numReplicas, 32, 0, stream>>>(tableDev, partials, chunks, cellEnergyDev, velDev, cellMassDev, out);
+    CUDA_CHECK(cudaGetLastError());
     std::vector<double> host(2*numReplicas);
-    cudaError_t err = cudaGetLastError();
-    if (err == cudaSuccess)
-        err = cudaMemcpyAsync(host.data(), out, sizeof(double)*2*numReplicas, cudaMemcpyDeviceToHost, stream);
-    if (err == cudaSuccess)
-        err = cudaStreamSynchronize(stream);
-    cudaFree(out);
-    CUDA_CHECK(err);
+    CUDA_CHECK(cudaMemcpyAsync(host.data(), out, sizeof(double)*2*numReplicas, cudaMemcpyDeviceToHost, stream));
+    CUDA_CHECK(cudaStreamSynchronize(stream));
     for (int r = 0; r < numReplicas; r++) {
         if (fluidKT)
             fluidKT[r] = host[2*r];

@@ -205,67 +205,82 @@ __device__ __forceinline__ void stencilAxes(const CouplingView& c, const double*
     }
 }
 
-// The node, weight and fluid velocity of stencil slot t = i*slots + s (particle i, slot s): the node and weight of
-// the slot (LBMStencils::axisWeights, LBMStencils.h:73-95) and the moments of the node pulled from the populations
-// (density, momentum after the momentum removal; a solid node has rho = 0).  centred: the velocity is
-// u~ = (j + h rho g)/rho (ReferenceLBMKernels.cpp:622, 773); explicit: u = j/rho (:539, :672).
+// The stencil slots t = i*slots + s of particle i by one warp: the node and weight of each slot (LBMStencils::axisWeights,
+// LBMStencils.h:73-95) and u = j/rho of the node pulled from the populations (after the momentum removal, :539, :672; a
+// solid node has rho = 0).  Lane 4 a + k < 12 forms entry k of axis a (index and weight, with axisWeights' merging of
+// repeated nodes), and each slot's lane takes its three entries by shuffles: a thread per slot formed all its particle's
+// entries again, nine to twelve kernel values in double with their roots, for the three that it uses (47 us per step of
+// 10,530 beads with the three-point stencil).  COHERENT: the positions were written by the same launch (a persistent
+// kernel): they are read through L2.
 template <typename T, typename R, bool COHERENT = false>
-__device__ __forceinline__ void stencilSlot(const T* __restrict__ A, const FluidView& f, const CouplingView& c,
-                                            const double* __restrict__ posIn, long long t, int remove, int centred,
-                                            int* slotNode, R* slotWeight, typename Vec4<R>::type* slotU) {
-    // COHERENT: the positions were written by the same launch (a persistent kernel): read them through L2.  The slots
-    // of all particles are fewer than 2^31: 32-bit division.
-    const int i = (int) t/c.slots, s = (int) t - i*c.slots;
-    double pos[3];
-    for (int a = 0; a < 3; a++)
-        pos[a] = COHERENT ? __ldcg(&posIn[3*i+a]) : posIn[3*i+a];
-    int size[3] = {c.nx, c.ny, c.nz};
-    int idx[3];
-    double w = 1.0;
+__device__ __forceinline__ void stencilParticle(const T* __restrict__ A, const FluidView& f, const CouplingView& c,
+                                                const double* __restrict__ pos, int i, int lane, int remove,
+                                                int* slotNode, R* slotWeight, typename Vec4<R>::type* slotU) {
+    const int axis = min(lane >> 2, 2), k = lane & 3;
+    const int size = axis == 0 ? c.nx : (axis == 1 ? c.ny : c.nz);
+    const double x = COHERENT ? __ldcg(&pos[3*i+axis]) : pos[3*i+axis];
+    const double s = latticeCoordinate(x, c.dx, size);
+    int index = -1 - k;
+    double weight = 0.0;
     if (c.stencil == LBM_STENCIL_NEAREST) {
-        // nearestNode (ReferenceLBMKernels.cpp:973-983): periodic wrap on every axis.
+        if (k == 0) {
+            index = ((int) floor(s + 0.5))%size;
+            weight = 1.0;
+        }
+    }
+    else if (k < c.width) {
+        const int first = c.stencil == LBM_STENCIL_THREEPOINT ? (int) floor(s + 0.5) - 1
+                        : (int) floor(s) - (c.stencil == LBM_STENCIL_KEYS ? 1 : 0);
+        weight = stencilKernel1(c.stencil, s - (first + k));
+        const int idx = first + k;
+        index = c.open[axis] ? min(max(idx, 0), size - 1) : ((idx%size) + size)%size;
+    }
+    // A node that the axis meets more than once keeps the sum of its weights in its first entry.
+    double merged = weight;
+    bool repeated = false;
+    for (int j = 0; j < 4; j++) {
+        const int other = __shfl_sync(0xffffffffu, index, (lane & ~3) + j);
+        const double w = __shfl_sync(0xffffffffu, weight, (lane & ~3) + j);
+        if (other == index && j < k)
+            repeated = true;
+        if (other == index && j > k)
+            merged += w;
+    }
+    weight = repeated ? 0.0 : merged;
+    const long long t0 = (long long) i*c.slots;
+    for (int s0 = 0; s0 < c.slots; s0 += 32) {
+        const int slot = s0 + lane, at = min(slot, c.slots - 1);
+        const int sub[3] = {at%c.width, (at/c.width)%c.width, at/(c.width*c.width)};
+        int idx[3];
+        double w = 1.0;
         for (int a = 0; a < 3; a++) {
-            double sc = latticeCoordinate(pos[a], c.dx, size[a]);
-            idx[a] = ((int) floor(sc + 0.5))%size[a];
+            idx[a] = __shfl_sync(0xffffffffu, index, 4*a + sub[a]);
+            w *= __shfl_sync(0xffffffffu, weight, 4*a + sub[a]);
         }
+        if (slot >= c.slots)
+            continue;
+        const long long node = idx[0] + (long long) c.nx*(idx[1] + (long long) c.ny*idx[2]);
+        double ux = 0, uy = 0, uz = 0, rho = 0;
+        if (w != 0.0 && !isSolid(c.solidMask, c.wordsPerRow, c.nx, node)) {
+            double dr, jx, jy, jz;
+            pullMomentsAt<T>(A, f, idx[0], idx[1], idx[2], dr, jx, jy, jz);
+            rho = 1.0 + dr;
+            if (remove) {
+                jx -= rho*f.stats->ucm[0];
+                jy -= rho*f.stats->ucm[1];
+                jz -= rho*f.stats->ucm[2];
+            }
+            ux = jx*(1.0/rho);
+            uy = jy*(1.0/rho);
+            uz = jz*(1.0/rho);
+        }
+        slotNode[t0 + slot] = (int) node;
+        slotWeight[t0 + slot] = (R) w;
+        slotU[t0 + slot] = Vec4<R>::make((R) ux, (R) uy, (R) uz, (R) rho);
     }
-    else {
-        int sub[3] = {s%c.width, (s/c.width)%c.width, s/(c.width*c.width)};
-        for (int a = 0; a < 3; a++) {
-            int index[4];
-            double weight[4];
-            axisWeights(c.stencil, c.width, latticeCoordinate(pos[a], c.dx, size[a]), size[a], c.open[a] != 0,
-                        index, weight);
-            idx[a] = index[sub[a]];
-            w *= weight[sub[a]];
-        }
-    }
-    long long node = idx[0] + (long long) c.nx*(idx[1] + (long long) c.ny*idx[2]);
-    slotNode[t] = (int) node;
-    slotWeight[t] = (R) w;
-    double ux = 0, uy = 0, uz = 0, rho = 0;
-    if (w != 0.0 && !isSolid(c.solidMask, c.wordsPerRow, c.nx, node)) {
-        double dr, jx, jy, jz;
-        pullMoments<T>(A, f, node, dr, jx, jy, jz);
-        rho = 1.0 + dr;
-        if (remove) {
-            jx -= rho*f.stats->ucm[0];
-            jy -= rho*f.stats->ucm[1];
-            jz -= rho*f.stats->ucm[2];
-        }
-        if (centred) {
-            jx += c.h*rho*c.g[0];
-            jy += c.h*rho*c.g[1];
-            jz += c.h*rho*c.g[2];
-        }
-        ux = jx*(1.0/rho);
-        uy = jy*(1.0/rho);
-        uz = jz*(1.0/rho);
-    }
-    slotU[t] = Vec4<R>::make((R) ux, (R) uy, (R) uz, (R) rho);
 }
 
-// The node and weight of stencil slot t, as stencilSlot (from the particle's axis indices and weights, computed once
+// The node and weight of stencil slot t, as stencilParticle (from the particle's axis indices and weights, computed once
 // per particle by stencilAxes), with the moments computed once per node: the first slot of a fluid node to claim it in
 // this pass (nodeStamp[node] set to `stamp`) pulls the node's moments into nodeU[node]; stencilGatherSlot then copies
 // them to every slot of the node.  The moments of a node are the same for all its slots, and overlapping stencils
