@@ -36,6 +36,28 @@ LbmStatus lbm_conv3d_status(void* stream);
  * default (2^24 polls).  No counterpart in the reference. */
 LbmStatus lbm_conv3d_set_wait_limit(long long polls);
 
+/* The network's passes between the convolutions, on channels-last BF16 volumes [batch][depth][height][width][channels]
+ * (channels multiples of 8, pointers aligned to 16 bytes); sizes are those of the larger volume.  Sums are formed in FP32
+ * and rounded once.
+ *   pool             y = mean of the 2 x 2 x 2 windows of x (a last odd plane is left out), and its gradient (dx of a left
+ *                    out plane is not written)
+ *   upsample_concat  y = the nearest 2x upsampling of x, then skip, along the channels (even sizes), and its gradients
+ *   relu_bias_grad   out = dy where y > 0 and 0 dy elsewhere, db[channels] += its sums over the voxels (FP32); with y NULL
+ *                    the sums of dy alone
+ *   input            the network's input for one solid mask (bytes): mask, inlet, xs[x], ys[y], zs[z] and three zeros per
+ *                    voxel */
+LbmStatus lbm_net_pool(const void* x, void* y, int batch, int depth, int height, int width, int channels, void* stream);
+LbmStatus lbm_net_pool_grad(const void* dy, void* dx, int batch, int depth, int height, int width, int channels,
+                            void* stream);
+LbmStatus lbm_net_upsample_concat(const void* x, const void* skip, void* y, int batch, int depth, int height, int width,
+                                  int channels, int skip_channels, void* stream);
+LbmStatus lbm_net_upsample_concat_grad(const void* dy, void* dx, void* dskip, int batch, int depth, int height, int width,
+                                       int channels, int skip_channels, void* stream);
+LbmStatus lbm_net_relu_bias_grad(const void* dy, const void* y, void* out, float* db, long long voxels, int channels,
+                                 void* stream);
+LbmStatus lbm_net_input(const void* mask, float inlet, const float* xs, const float* ys, const float* zs, void* out,
+                        int depth, int height, int width, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

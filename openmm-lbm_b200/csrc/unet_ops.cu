@@ -1,0 +1,264 @@
+// The learned warm start's passes between the convolutions (include/lbm_b200_warmstart.h), on channels-last BF16 volumes
+// [n][d][h][w][c] with 8 channels (16 bytes) per thread: pooling, upsampling into the concatenation with the skip, their
+// gradients, the gradient through a layer's ReLU with its bias's, and the network's input.  They are bound by memory;
+// each reads and writes every volume once, in the layout the convolutions use.  The library passes that they stand in for
+// worked in planar order between layout copies.  Per training step on two 64 x 64 x 128 volumes: upsampling with the
+// concatenation 43 us (262, and the copies around it), its gradients 37 us (140 and copies), the ReLU's and biases'
+// gradients of 15 layers 138 us (980 in five passes), pooling 9 us (56), the input 5 us per mask (twelve launches).
+#include "lbm_b200_warmstart.h"
+#include "lbm_internal.h"
+#include <cuda_bf16.h>
+#include <algorithm>
+#include <string>
+
+namespace {
+
+constexpr int kThreads = 256;
+
+struct Row {
+    int n, z, y;
+};
+__device__ __forceinline__ Row rowOf(unsigned row, int depth, int height) {
+    Row r;
+    r.y = (int) (row%(unsigned) height);
+    row /= (unsigned) height;
+    r.z = (int) (row%(unsigned) depth);
+    r.n = (int) (row/(unsigned) depth);
+    return r;
+}
+
+// The 16-byte word of channel group g of voxel (z, y, x).
+__device__ __forceinline__ size_t wordAt(int n, int z, int y, int x, int D, int H, int W, int groups, int g) {
+    return ((((size_t) n*D + z)*H + y)*W + x)*groups + g;
+}
+
+__device__ __forceinline__ void unpack(uint4 v, float (&f)[8]) {
+    const unsigned w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        f[2*i] = __uint_as_float(w[i] << 16);
+        f[2*i+1] = __uint_as_float(w[i] & 0xFFFF0000u);
+    }
+}
+__device__ __forceinline__ uint4 pack(const float (&f)[8]) {
+    unsigned w[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(f[2*i], f[2*i+1]);
+        w[i] = *reinterpret_cast<const unsigned*>(&h);
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// Sums of 8 children in the order of the window (z, y, x), in float, rounded once.
+__device__ __forceinline__ uint4 sumChildren(const uint4* __restrict__ v, int n, int z, int y, int x, int D, int H, int W,
+                                             int groups, int g, float scale) {
+    uint4 word[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+        word[i] = __ldg(v + wordAt(n, 2*z + i/4, 2*y + i/2%2, 2*x + i%2, D, H, W, groups, g));
+    float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        float f[8];
+        unpack(word[i], f);
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            s[k] += f[k];
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+        s[k] *= scale;
+    return pack(s);
+}
+
+// y [n][d][h][w] = mean of x's 2 x 2 x 2 windows; a block per row of y.
+__global__ void __launch_bounds__(kThreads)
+poolKernel(const uint4* __restrict__ x, uint4* __restrict__ y, int D, int H, int W, int groups) {
+    const int d = D/2, h = H/2, w = W/2;
+    const Row r = rowOf(blockIdx.x, d, h);
+    for (int i = threadIdx.x; i < w*groups; i += blockDim.x) {
+        const int xx = i/groups, g = i - xx*groups;
+        y[(size_t) blockIdx.x*w*groups + i] = sumChildren(x, r.n, r.z, r.y, xx, D, H, W, groups, g, 0.125f);
+    }
+}
+
+// The gradient of the pooling: dx = dy/8 in every window's voxels (D, H, W of dx, even or with an untouched last plane).
+__global__ void __launch_bounds__(kThreads)
+poolGradKernel(const uint4* __restrict__ dy, uint4* __restrict__ dx, int D, int H, int W, int groups) {
+    const int d = D/2, h = H/2, w = W/2;
+    const Row r = rowOf(blockIdx.x, d, h);
+    for (int i = threadIdx.x; i < w*groups; i += blockDim.x) {
+        const int xx = i/groups, g = i - xx*groups;
+        float f[8];
+        unpack(__ldg(dy + (size_t) blockIdx.x*w*groups + i), f);
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            f[k] *= 0.125f;
+        const uint4 v = pack(f);
+#pragma unroll
+        for (int c = 0; c < 8; c++)
+            dx[wordAt(r.n, 2*r.z + c/4, 2*r.y + c/2%2, 2*xx + c%2, D, H, W, groups, g)] = v;
+    }
+}
+
+// y = [nearest 2x upsampling of x, skip] along the channels; a block per row of y (D, H, W).
+__global__ void __launch_bounds__(kThreads)
+upsampleConcatKernel(const uint4* __restrict__ x, const uint4* __restrict__ skip, uint4* __restrict__ y, int D, int H, int W,
+                     int groupsX, int groupsSkip) {
+    const int groups = groupsX + groupsSkip;
+    const Row r = rowOf(blockIdx.x, D, H);
+    for (int i = threadIdx.x; i < W*groups; i += blockDim.x) {
+        const int xx = i/groups, g = i - xx*groups;
+        y[(size_t) blockIdx.x*W*groups + i] = g < groupsX
+            ? __ldg(x + wordAt(r.n, r.z/2, r.y/2, xx/2, D/2, H/2, W/2, groupsX, g))
+            : __ldg(skip + ((size_t) blockIdx.x*W + xx)*groupsSkip + (g - groupsX));
+    }
+}
+
+// Its gradients: dx the sums of dy over the upsampled voxels, dskip the other channels; a block per row of dx.
+__global__ void __launch_bounds__(kThreads)
+upsampleConcatGradKernel(const uint4* __restrict__ dy, uint4* __restrict__ dx, uint4* __restrict__ dskip, int D, int H, int W,
+                         int groupsX, int groupsSkip) {
+    const int groups = groupsX + groupsSkip, d = D/2, h = H/2, w = W/2;
+    const Row r = rowOf(blockIdx.x, d, h);
+    for (int i = threadIdx.x; i < w*groupsX; i += blockDim.x) {
+        const int xx = i/groupsX, g = i - xx*groupsX;
+        dx[(size_t) blockIdx.x*w*groupsX + i] = sumChildren(dy, r.n, r.z, r.y, xx, D, H, W, groups, g, 1.0f);
+    }
+    for (int i = threadIdx.x; i < 4*W*groupsSkip; i += blockDim.x) {
+        const int line = i/(W*groupsSkip), j = i - line*W*groupsSkip, xx = j/groupsSkip, g = j - xx*groupsSkip;
+        const int z = 2*r.z + line/2, y = 2*r.y + line%2;
+        dskip[wordAt(r.n, z, y, xx, D, H, W, groupsSkip, g)] = __ldg(dy + wordAt(r.n, z, y, xx, D, H, W, groups, groupsX + g));
+    }
+}
+
+// The gradient of a layer's output before its ReLU, dy (y > 0) (y == nullptr: no ReLU, and out is not written), and its
+// sums over the voxels added to db: a thread keeps one channel group and adds up its voxels, a block its threads.
+__global__ void __launch_bounds__(kThreads)
+reluBiasGradKernel(const uint4* __restrict__ dy, const uint4* __restrict__ y, uint4* __restrict__ out, float* __restrict__ db,
+                   size_t voxels, int groups) {
+    extern __shared__ float sums[];                       // [threads][8]
+    const int lanes = kThreads/groups;                    // voxels a block takes at a time
+    const int g = threadIdx.x%groups, lane = threadIdx.x/groups;
+    float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (lane < lanes)
+        for (size_t v = (size_t) blockIdx.x*lanes + lane; v < voxels; v += (size_t) gridDim.x*lanes) {
+            const uint4 word = __ldg(dy + v*groups + g);
+            float f[8];
+            unpack(word, f);
+            if (y != nullptr) {
+                float a[8];
+                unpack(__ldg(y + v*groups + g), a);
+#pragma unroll
+                for (int k = 0; k < 8; k++)
+                    f[k] = a[k] > 0.0f ? f[k] : 0.0f*f[k];
+                out[v*groups + g] = pack(f);
+            }
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+                s[k] += f[k];
+        }
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+        sums[threadIdx.x*8 + k] = s[k];
+    __syncthreads();
+    for (int c = threadIdx.x; c < 8*groups; c += blockDim.x) {
+        float total = 0;
+        for (int l = 0; l < lanes; l++)
+            total += sums[(l*groups + c/8)*8 + c%8];
+        atomicAdd(db + c, total);
+    }
+}
+
+// The network's input for one mask: solid, scaled inlet and the coordinates along x, y, z, then zeros; 8 channels a voxel.
+__global__ void __launch_bounds__(kThreads)
+inputKernel(const unsigned char* __restrict__ mask, float inlet, const float* __restrict__ xs, const float* __restrict__ ys,
+            const float* __restrict__ zs, uint4* __restrict__ out, int H, int W) {
+    const float y = ys[blockIdx.x%(unsigned) H], z = zs[blockIdx.x/(unsigned) H];
+    for (int x = threadIdx.x; x < W; x += blockDim.x) {
+        const size_t v = (size_t) blockIdx.x*W + x;
+        const float f[8] = {mask[v] ? 1.0f : 0.0f, inlet, xs[x], y, z, 0.0f, 0.0f, 0.0f};
+        out[v] = pack(f);
+    }
+}
+
+LbmStatus invalid(const char* message) {
+    lbm::setLastError(message);
+    return LBM_ERR_INVALID_ARGUMENT;
+}
+
+LbmStatus launched(const char* name) {
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess)
+        return LBM_OK;
+    lbm::setLastError(std::string(name) + ": " + cudaGetErrorString(e));
+    return LBM_ERR_CUDA;
+}
+
+// A block per row: their number must fit a grid.
+bool rowsFit(int batch, int depth, int height) {
+    return batch > 0 && depth > 0 && height > 0 && (long long) batch*depth*height < (1LL << 31);
+}
+
+} // namespace
+
+extern "C" {
+
+LbmStatus lbm_net_pool(const void* x, void* y, int batch, int depth, int height, int width, int channels, void* stream) {
+    if (!x || !y || channels <= 0 || channels%8 != 0 || !rowsFit(batch, depth/2, height/2) || width < 2)
+        return invalid("lbm_net_pool: null pointer, empty volume or channels not a multiple of 8");
+    poolKernel<<<(unsigned) (batch*(depth/2)*(height/2)), kThreads, 0, (cudaStream_t) stream>>>(
+        (const uint4*) x, (uint4*) y, depth, height, width, channels/8);
+    return launched("lbm_net_pool");
+}
+
+LbmStatus lbm_net_pool_grad(const void* dy, void* dx, int batch, int depth, int height, int width, int channels, void* stream) {
+    if (!dy || !dx || channels <= 0 || channels%8 != 0 || !rowsFit(batch, depth/2, height/2) || width < 2)
+        return invalid("lbm_net_pool_grad: null pointer, empty volume or channels not a multiple of 8");
+    poolGradKernel<<<(unsigned) (batch*(depth/2)*(height/2)), kThreads, 0, (cudaStream_t) stream>>>(
+        (const uint4*) dy, (uint4*) dx, depth, height, width, channels/8);
+    return launched("lbm_net_pool_grad");
+}
+
+LbmStatus lbm_net_upsample_concat(const void* x, const void* skip, void* y, int batch, int depth, int height, int width,
+                                  int channels, int skip_channels, void* stream) {
+    if (!x || !skip || !y || channels <= 0 || channels%8 != 0 || skip_channels <= 0 || skip_channels%8 != 0 ||
+        !rowsFit(batch, depth, height) || width <= 0 || depth%2 != 0 || height%2 != 0 || width%2 != 0)
+        return invalid("lbm_net_upsample_concat: null pointer, odd or empty volume or channels not a multiple of 8");
+    upsampleConcatKernel<<<(unsigned) (batch*depth*height), kThreads, 0, (cudaStream_t) stream>>>(
+        (const uint4*) x, (const uint4*) skip, (uint4*) y, depth, height, width, channels/8, skip_channels/8);
+    return launched("lbm_net_upsample_concat");
+}
+
+LbmStatus lbm_net_upsample_concat_grad(const void* dy, void* dx, void* dskip, int batch, int depth, int height, int width,
+                                       int channels, int skip_channels, void* stream) {
+    if (!dy || !dx || !dskip || channels <= 0 || channels%8 != 0 || skip_channels <= 0 || skip_channels%8 != 0 ||
+        !rowsFit(batch, depth, height) || width <= 0 || depth%2 != 0 || height%2 != 0 || width%2 != 0)
+        return invalid("lbm_net_upsample_concat_grad: null pointer, odd or empty volume or channels not a multiple of 8");
+    upsampleConcatGradKernel<<<(unsigned) (batch*(depth/2)*(height/2)), kThreads, 0, (cudaStream_t) stream>>>(
+        (const uint4*) dy, (uint4*) dx, (uint4*) dskip, depth, height, width, channels/8, skip_channels/8);
+    return launched("lbm_net_upsample_concat_grad");
+}
+
+LbmStatus lbm_net_relu_bias_grad(const void* dy, const void* y, void* out, float* db, long long voxels, int channels,
+                                 void* stream) {
+    if (!dy || !db || (y && !out) || voxels <= 0 || channels <= 0 || channels%8 != 0 || channels > 8*kThreads)
+        return invalid("lbm_net_relu_bias_grad: null pointer, empty volume or channels not a multiple of 8");
+    const int groups = channels/8, lanes = kThreads/groups;
+    const long long blocks = std::min<long long>(592, (voxels + lanes - 1)/lanes);
+    reluBiasGradKernel<<<(unsigned) blocks, kThreads, kThreads*8*sizeof(float), (cudaStream_t) stream>>>(
+        (const uint4*) dy, (const uint4*) y, (uint4*) out, db, (size_t) voxels, groups);
+    return launched("lbm_net_relu_bias_grad");
+}
+
+LbmStatus lbm_net_input(const void* mask, float inlet, const float* xs, const float* ys, const float* zs, void* out,
+                        int depth, int height, int width, void* stream) {
+    if (!mask || !xs || !ys || !zs || !out || !rowsFit(1, depth, height) || width <= 0)
+        return invalid("lbm_net_input: null pointer or empty volume");
+    inputKernel<<<(unsigned) (depth*height), kThreads, 0, (cudaStream_t) stream>>>((const unsigned char*) mask, inlet, xs, ys,
+                                                                                  zs, (uint4*) out, height, width);
+    return launched("lbm_net_input");
+}
+
+} // extern "C"

@@ -37,6 +37,13 @@ _SIGNATURES = {
                                               ctypes.c_void_p]),
     'lbm_conv3d_status': (ctypes.c_int, [ctypes.c_void_p]),
     'lbm_conv3d_set_wait_limit': (ctypes.c_int, [ctypes.c_longlong]),
+    'lbm_net_pool': (ctypes.c_int, [ctypes.c_void_p]*2 + [ctypes.c_int]*5 + [ctypes.c_void_p]),
+    'lbm_net_pool_grad': (ctypes.c_int, [ctypes.c_void_p]*2 + [ctypes.c_int]*5 + [ctypes.c_void_p]),
+    'lbm_net_upsample_concat': (ctypes.c_int, [ctypes.c_void_p]*3 + [ctypes.c_int]*6 + [ctypes.c_void_p]),
+    'lbm_net_upsample_concat_grad': (ctypes.c_int, [ctypes.c_void_p]*3 + [ctypes.c_int]*6 + [ctypes.c_void_p]),
+    'lbm_net_relu_bias_grad': (ctypes.c_int, [ctypes.c_void_p]*4 + [ctypes.c_longlong, ctypes.c_int, ctypes.c_void_p]),
+    'lbm_net_input': (ctypes.c_int, [ctypes.c_void_p, ctypes.c_float] + [ctypes.c_void_p]*4 + [ctypes.c_int]*3 +
+                      [ctypes.c_void_p]),
 }
 
 INLET_SCALE = 0.02
@@ -116,13 +123,86 @@ class Conv3dFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, w16, y = ctx.saved_tensors
-        dy = _volume(dy.to(torch.bfloat16))
-        if ctx.relu:
-            dy = _volume(dy*(y > 0).to(dy.dtype))
+        dy, db = relu_bias_grad(dy, y)
         dx = conv3d_input_grad(dy, w16) if ctx.needs_input_grad[0] else None
         dw = conv3d_weight_grad(x, dy)
-        db = dy.float().sum(dim=(0, 2, 3, 4))
         return dx, dw, db, None
+
+
+def _empty_volume(like, channels, d, h, w):
+    return torch.empty((like.shape[0], channels, d, h, w), device=like.device, dtype=torch.bfloat16,
+                       memory_format=torch.channels_last_3d)
+
+
+def relu_bias_grad(dy, y=None):
+    """The gradient of a convolution's output before its ReLU (y, the layer's output; None without one), in BF16, and
+    its sums over the voxels in FP32: the bias's gradient."""
+    lib = _lib()
+    dy = _volume(dy.to(torch.bfloat16))
+    channels = dy.shape[1]
+    db = torch.zeros(channels, device=dy.device, dtype=torch.float32)
+    out = dy
+    if y is not None:
+        y = _volume(y)
+        out = torch.empty_like(dy)
+    check(lib.lbm_net_relu_bias_grad(dy.data_ptr(), y.data_ptr() if y is not None else None, out.data_ptr(), db.data_ptr(),
+                                     dy.numel()//channels, channels, _stream()), lib)
+    return out, db
+
+
+class Pool2(torch.autograd.Function):
+    """Mean over 2 x 2 x 2 windows of a channels-last BF16 volume (as avg_pool3d)."""
+
+    @staticmethod
+    def forward(ctx, x):
+        lib = _lib()
+        x = _volume(x)
+        n, c, d, h, w = x.shape
+        ctx.size = (d, h, w)
+        y = _empty_volume(x, c, d//2, h//2, w//2)
+        check(lib.lbm_net_pool(x.data_ptr(), y.data_ptr(), n, d, h, w, c, _stream()), lib)
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        lib = _lib()
+        dy = _volume(dy.to(torch.bfloat16))
+        d, h, w = ctx.size
+        n, c = dy.shape[:2]
+        dx = _empty_volume(dy, c, d, h, w)
+        if d % 2 or h % 2 or w % 2:
+            dx.zero_()
+        check(lib.lbm_net_pool_grad(dy.data_ptr(), dx.data_ptr(), n, d, h, w, c, _stream()), lib)
+        return dx
+
+
+class UpsampleConcat(torch.autograd.Function):
+    """Nearest 2x upsampling of x concatenated with the skip along the channels (channels-last BF16 volumes)."""
+
+    @staticmethod
+    def forward(ctx, x, skip):
+        lib = _lib()
+        x, skip = _volume(x), _volume(skip)
+        n, c, d, h, w = x.shape
+        if skip.shape[0] != n or tuple(skip.shape[2:]) != (2*d, 2*h, 2*w):
+            raise RuntimeError('the skip (%s) does not match the upsampled volume (%s)' %
+                               (tuple(skip.shape), (n, c, 2*d, 2*h, 2*w)))
+        ctx.channels = (c, skip.shape[1])
+        y = _empty_volume(x, c + skip.shape[1], 2*d, 2*h, 2*w)
+        check(lib.lbm_net_upsample_concat(x.data_ptr(), skip.data_ptr(), y.data_ptr(), n, 2*d, 2*h, 2*w, c, skip.shape[1],
+                                          _stream()), lib)
+        return y
+
+    @staticmethod
+    def backward(ctx, dy):
+        lib = _lib()
+        dy = _volume(dy.to(torch.bfloat16))
+        n, _, d, h, w = dy.shape
+        c, cs = ctx.channels
+        dx, dskip = _empty_volume(dy, c, d//2, h//2, w//2), _empty_volume(dy, cs, d, h, w)
+        check(lib.lbm_net_upsample_concat_grad(dy.data_ptr(), dx.data_ptr(), dskip.data_ptr(), n, d, h, w, c, cs, _stream()),
+              lib)
+        return dx, dskip
 
 
 class WarmStartNet(torch.nn.Module):
@@ -167,10 +247,9 @@ class WarmStartNet(torch.nn.Module):
             i += 2
             if level < levels - 1:
                 skips.append(h)
-                h = _volume(torch.nn.functional.avg_pool3d(h, 2))
+                h = Pool2.apply(h)
         for level in range(levels - 2, -1, -1):
-            h = torch.nn.functional.interpolate(h, scale_factor=2, mode='nearest')
-            h = _volume(torch.cat([h, skips[level]], dim=1))
+            h = UpsampleConcat.apply(h, skips[level])
             h = self._conv(i + 1, self._conv(i, h))
             i += 2
         return self._conv(i, h, relu=False)[:, :self.out_channels]
@@ -218,6 +297,16 @@ def network_input(masks, inlet=0.02):
     n = len(masks)
     nz, ny, nx = masks[0].shape
     dev = masks[0].device
+    if all(m.is_cuda and m.dtype == torch.bool and tuple(m.shape) == (nz, ny, nx) and m.device == dev for m in masks):
+        lib = _lib()
+        axes = [torch.linspace(0, 1, k, device=dev) for k in (nx, ny, nz)]
+        x = torch.empty((n, IN_CHANNELS, nz, ny, nx), device=dev, dtype=torch.bfloat16,
+                        memory_format=torch.channels_last_3d)
+        for i, m in enumerate(masks):
+            m = m.contiguous()
+            check(lib.lbm_net_input(m.data_ptr(), inlet/INLET_SCALE, axes[0].data_ptr(), axes[1].data_ptr(),
+                                    axes[2].data_ptr(), x[i].data_ptr(), nz, ny, nx, _stream()), lib)
+        return x
     x = torch.zeros((n, IN_CHANNELS, nz, ny, nx), device=dev, dtype=torch.float32)
     zz = torch.linspace(0, 1, nz, device=dev).view(nz, 1, 1)
     yy = torch.linspace(0, 1, ny, device=dev).view(1, ny, 1)
