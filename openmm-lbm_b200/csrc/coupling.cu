@@ -42,18 +42,26 @@ const int kThreads = 256;
 // The stencil pass: the axis indices and weights of each particle, then one thread per (particle, stencil slot) in
 // two passes: nodes, weights and the moments of each node once, then the moments of every slot.
 // One thread per particle: the node indices and weights of its stencil on each axis, and the first index on each.
+// The node indices and weights of every particle's stencil on each axis (entries past the width: index -1, weight 0), 16
+// threads per particle, one per entry: with a thread per particle its twelve kernel values in double came one after
+// another (8.1 -> 3.0 us for 6,400 particles with Keys).
 __global__ void stencilAxesKernel(CouplingView c, const double* __restrict__ pos, int4* axisIndex, double2* axisWeight,
                                   int4* firstIndex) {
-    for (int i = blockIdx.x*blockDim.x + threadIdx.x; i < c.np; i += gridDim.x*blockDim.x) {
-        int index[3][4];
-        double weight[3][4];
-        stencilAxes(c, pos, i, index, weight);
-        for (int a = 0; a < 3; a++) {
-            axisIndex[3*i + a] = make_int4(index[a][0], index[a][1], index[a][2], index[a][3]);
-            axisWeight[6*i + 2*a] = make_double2(weight[a][0], weight[a][1]);
-            axisWeight[6*i + 2*a + 1] = make_double2(weight[a][2], weight[a][3]);
+    const int lane = threadIdx.x & 31, half = lane >> 4, entry = lane & 15;
+    const int warps = (gridDim.x*blockDim.x) >> 5;
+    for (int w = (blockIdx.x*blockDim.x + threadIdx.x) >> 5; 2*w < c.np; w += warps) {
+        const int i = min(2*w + half, c.np - 1);
+        int index;
+        double weight;
+        stencilEntry<false>(c, pos, i, lane, index, weight);
+        if (entry < 12 && 2*w + half < c.np) {
+            reinterpret_cast<int*>(axisIndex)[12*(size_t) i + entry] = max(index, -1);
+            reinterpret_cast<double*>(axisWeight)[12*(size_t) i + entry] = weight;
+            if ((entry & 3) == 0)
+                reinterpret_cast<int*>(firstIndex)[4*(size_t) i + (entry >> 2)] = index;
         }
-        firstIndex[i] = make_int4(index[0][0], index[1][0], index[2][0], 0);
+        else if (entry == 12 && 2*w + half < c.np)
+            reinterpret_cast<int*>(firstIndex)[4*(size_t) i + 3] = 0;
     }
 }
 
@@ -176,32 +184,38 @@ struct CgBuffers {
 
 // Block sum of a record (thread values v) into partials[block]; after a grid barrier (by the caller) every block adds
 // the records of all blocks in block order, so every block gets the same result, bit for bit.
-__device__ void blockSumStore(double v[kPartial], double* partials) {
+// (N components: those that the phase sums), by warps and then a warp per component.
+template <int N>
+__device__ __forceinline__ void blockSumStore(double (&v)[N], double* partials) {
+    static_assert(N <= kPartial, "a record holds kPartial values");
     __shared__ double red[32][kPartial];
-    int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int k = 0; k < kPartial; k++)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+#pragma unroll
+    for (int k = 0; k < N; k++)
         v[k] = warpSum(v[k]);
     if (lane == 0)
-        for (int k = 0; k < kPartial; k++)
+#pragma unroll
+        for (int k = 0; k < N; k++)
             red[warp][k] = v[k];
     __syncthreads();
-    if (threadIdx.x < kPartial) {
-        double s = 0;
-        for (int w = 0; w < (int) blockDim.x/32; w++)
-            s += red[w][threadIdx.x];
-        partials[kPartial*blockIdx.x + threadIdx.x] = s;
+    for (int k = warp; k < N; k += warps) {
+        const double s = warpSum(lane < warps ? red[lane][k] : 0.0);
+        if (lane == 0)
+            partials[kPartial*blockIdx.x + k] = s;
     }
     __syncthreads();
 }
 
-__device__ void reducePartials(const double* partials, int count, double out[kPartial]) {
+template <int N>
+__device__ __forceinline__ void reducePartials(const double* partials, int count, double (&out)[N]) {
     // Warp k sums component k over the blocks (lanes strided over the records, then a fixed tree), so every block
     // gets the same result, bit for bit.  The records were written by other blocks before a grid barrier: loads bypass
     // L1.
     __shared__ double total[kPartial];
     const int lane = threadIdx.x & 31;
-    for (int k = threadIdx.x >> 5; k < kPartial; k += blockDim.x >> 5) {
+    for (int k = threadIdx.x >> 5; k < N; k += blockDim.x >> 5) {
         double s = 0;
+#pragma unroll 5
         for (int r = lane; r < count; r += 32)
             s += __ldcg(partials + kPartial*r + k);
         s = warpSum(s);
@@ -209,7 +223,8 @@ __device__ void reducePartials(const double* partials, int count, double out[kPa
             total[k] = s;
     }
     __syncthreads();
-    for (int k = 0; k < kPartial; k++)
+#pragma unroll
+    for (int k = 0; k < N; k++)
         out[k] = total[k];
     __syncthreads();
 }
@@ -313,7 +328,7 @@ centeredStencilKernel(FluidView f, CouplingView c, const double* __restrict__ ve
     if (!gridSync(b.barrier, b.status, b.pollLimit))
         return;
     // r = rhs - A F, z = r/diag, p = z; r.z, the norm of the right-hand side and r.r per component.
-    double acc[kPartial] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+    double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     for (int i = firstWarp; i < c.np; i += warps) {
         double g[3];
         gather(i, g);
@@ -338,7 +353,7 @@ centeredStencilKernel(FluidView f, CouplingView c, const double* __restrict__ ve
         return;
     for (int i = firstWarp; i < c.np; i += warps)
         clearSpread(i);
-    double tot[kPartial];
+    double tot[9];
     reducePartials(b.partials[1], gridDim.x, tot);
     double rz[3] = {tot[0], tot[1], tot[2]}, norm[3] = {tot[3], tot[4], tot[5]}, residual[3] = {tot[6], tot[7], tot[8]};
     int iteration = 0;
@@ -368,7 +383,7 @@ centeredStencilKernel(FluidView f, CouplingView c, const double* __restrict__ ve
             spreadP(i, b.p);
         if (!gridSync(b.barrier, b.status, b.pollLimit))
             return;
-        double acc3[kPartial] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+        double acc3[3] = {0, 0, 0}, pAp[3];
         for (int i = firstWarp; i < c.np; i += warps) {
             double g[3];
             gather(i, g);
@@ -385,11 +400,11 @@ centeredStencilKernel(FluidView f, CouplingView c, const double* __restrict__ ve
         blockSumStore(acc3, b.partials[0]);
         if (!gridSync(b.barrier, b.status, b.pollLimit))
             return;
-        reducePartials(b.partials[0], gridDim.x, tot);
+        reducePartials(b.partials[0], gridDim.x, pAp);
         double alpha[3];
         for (int d = 0; d < 3; d++)
-            alpha[d] = (tot[d] > 0 ? rz[d]/tot[d] : 0.0);
-        double acc4[kPartial] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+            alpha[d] = (pAp[d] > 0 ? rz[d]/pAp[d] : 0.0);
+        double acc4[6] = {0, 0, 0, 0, 0, 0}, sums[6];
         for (int i = firstWarp; i < c.np; i += warps) {
             clearSpread(i);
             if (lane == 0) {
@@ -408,12 +423,12 @@ centeredStencilKernel(FluidView f, CouplingView c, const double* __restrict__ ve
         blockSumStore(acc4, b.partials[1]);
         if (!gridSync(b.barrier, b.status, b.pollLimit))
             return;
-        reducePartials(b.partials[1], gridDim.x, tot);
+        reducePartials(b.partials[1], gridDim.x, sums);
         double beta[3];
         for (int d = 0; d < 3; d++) {
-            beta[d] = (rz[d] > 0 ? tot[d]/rz[d] : 0.0);
-            rz[d] = tot[d];
-            residual[d] = tot[3+d];
+            beta[d] = (rz[d] > 0 ? sums[d]/rz[d] : 0.0);
+            rz[d] = sums[d];
+            residual[d] = sums[3+d];
         }
         if (lane == 0)
             for (int i = firstWarp; i < c.np; i += warps)
@@ -775,7 +790,7 @@ centeredSparseKernel(FluidView f, CouplingView c, const double* __restrict__ vel
     if (!gridSync(b.barrier, b.status, b.pollLimit))
         return;
     // r = rhs - A F, z = r/diag, p = z; r.z, the norm of the right-hand side and r.r per component.
-    double acc[kPartial] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+    double acc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     for (int base = rowBegin; base < rowEnd; base += blockDim.x/kProductLanes) {
         const int i = base + threadIdx.x/kProductLanes;
         double g3[3];
@@ -799,7 +814,7 @@ centeredSparseKernel(FluidView f, CouplingView c, const double* __restrict__ vel
     blockSumStore(acc, b.partials[1]);
     if (!gridSync(b.barrier, b.status, b.pollLimit))
         return;
-    double tot[kPartial];
+    double tot[9];
     reducePartials(b.partials[1], gridDim.x, tot);
     double rz[3] = {tot[0], tot[1], tot[2]}, norm[3] = {tot[3], tot[4], tot[5]}, residual[3] = {tot[6], tot[7], tot[8]};
     double beta[3] = {0, 0, 0};
@@ -819,7 +834,7 @@ centeredSparseKernel(FluidView f, CouplingView c, const double* __restrict__ vel
             break;
         }
         // p = z + beta p and A p = A z + beta A p (p = z at the first iteration), with p.Ap.
-        double acc3[kPartial] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+        double acc3[3] = {0, 0, 0}, pAp[3];
         for (int base = rowBegin; base < rowEnd; base += blockDim.x/kProductLanes) {
             const int i = base + threadIdx.x/kProductLanes;
             double g3[3];
@@ -843,11 +858,11 @@ centeredSparseKernel(FluidView f, CouplingView c, const double* __restrict__ vel
         blockSumStore(acc3, b.partials[0]);
         if (!gridSync(b.barrier, b.status, b.pollLimit))
             return;
-        reducePartials(b.partials[0], gridDim.x, tot);
+        reducePartials(b.partials[0], gridDim.x, pAp);
         double alpha[3];
         for (int d = 0; d < 3; d++)
-            alpha[d] = (tot[d] > 0 ? rz[d]/tot[d] : 0.0);
-        double acc4[kPartial] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+            alpha[d] = (pAp[d] > 0 ? rz[d]/pAp[d] : 0.0);
+        double acc4[6] = {0, 0, 0, 0, 0, 0}, sums[6];
         for (int i = rowBegin + threadIdx.x; i < rowEnd; i += blockDim.x) {
             double diag = b.diag[i];
             for (int d = 0; d < 3; d++) {
@@ -863,11 +878,11 @@ centeredSparseKernel(FluidView f, CouplingView c, const double* __restrict__ vel
         blockSumStore(acc4, b.partials[1]);
         if (!gridSync(b.barrier, b.status, b.pollLimit))
             return;
-        reducePartials(b.partials[1], gridDim.x, tot);
+        reducePartials(b.partials[1], gridDim.x, sums);
         for (int d = 0; d < 3; d++) {
-            beta[d] = (rz[d] > 0 ? tot[d]/rz[d] : 0.0);
-            rz[d] = tot[d];
-            residual[d] = tot[3+d];
+            beta[d] = (rz[d] > 0 ? sums[d]/rz[d] : 0.0);
+            rz[d] = sums[d];
+            residual[d] = sums[3+d];
         }
     }
     if (firstWarp == 0 && lane == 0)
@@ -1100,7 +1115,8 @@ CouplingEngine::CouplingEngine(const LbmLatticeParameters& l, FluidEngine& f, co
             dev->sparseGrid = (int) std::max(1LL, std::min(std::min(wantedSolve, (long long) std::max(1, perSM)*sms),
                                                           (long long) dev->cgGrid));
         }
-        CUDA_CHECK(cudaMallocHost(&pinned, v3));
+        CUDA_CHECK(cudaMallocHost(&pinned, v3 + 4*sizeof(int)));
+        statusHost = reinterpret_cast<int*>(pinned + 3*(size_t) np);
         CUDA_CHECK(cudaStreamSynchronize(stream));
     }
     catch (...) {
@@ -1154,17 +1170,26 @@ void CouplingEngine::setParameters(const LbmLatticeParameters& l) {
     lattice = l;
 }
 
-void CouplingEngine::load(const LbmParticleArrays* p, bool withForces) {
-    size_t v3 = sizeof(double)*3*(size_t) np;
-    cudaMemcpyKind kind = p->memory == LBM_MEMORY_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-    CUDA_CHECK(cudaMemcpyAsync(posDev, p->positions, v3, kind, stream));
-    CUDA_CHECK(cudaMemcpyAsync(velDev, p->velocities, v3, kind, stream));
+void CouplingEngine::load(const LbmParticleArrays* p, bool withForces, bool withPositions) {
+    const size_t v3 = sizeof(double)*3*(size_t) np;
+    const bool onDevice = p->memory == LBM_MEMORY_DEVICE;
+    if (withPositions)
+        CUDA_CHECK(cudaMemcpyAsync(posDev, p->positions, v3, onDevice ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, stream));
+    // The kernels of this call read device arrays in place (they run on the stream of the copies they replace).
+    velIn = onDevice ? p->velocities : velDev;
+    forceIn = onDevice && withForces ? p->forces : forceInDev;
+    if (onDevice)
+        return;
+    CUDA_CHECK(cudaMemcpyAsync(velDev, p->velocities, v3, cudaMemcpyHostToDevice, stream));
     if (withForces)
-        CUDA_CHECK(cudaMemcpyAsync(forceInDev, p->forces, v3, kind, stream));
+        CUDA_CHECK(cudaMemcpyAsync(forceInDev, p->forces, v3, cudaMemcpyHostToDevice, stream));
 }
 
 void CouplingEngine::reflect(const LbmParticleArrays* p, double wallMomentum[3]) {
-    load(p, false);
+    const size_t v3 = sizeof(double)*3*(size_t) np;
+    const cudaMemcpyKind in = p->memory == LBM_MEMORY_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+    CUDA_CHECK(cudaMemcpyAsync(posDev, p->positions, v3, in, stream));
+    CUDA_CHECK(cudaMemcpyAsync(velDev, p->velocities, v3, in, stream));
     const FluidView& f = fluid.deviceView();
     CouplingView c = makeCouplingView(lattice, f, np, 1, massDev);
     CUDA_CHECK(cudaMemsetAsync(dev->reflectWall, 0, sizeof(double)*3, stream));
@@ -1172,9 +1197,8 @@ void CouplingEngine::reflect(const LbmParticleArrays* p, double wallMomentum[3])
     reflectKernel<<<std::max(1, std::min(1184, (np + kThreads - 1)/kThreads)), kThreads, 0, stream>>>(c, posDev, velDev, cellMass, dev->reflectWall);
     CUDA_CHECK(cudaGetLastError());
     fluid.launches++;
-    size_t v3 = sizeof(double)*3*(size_t) np;
-    cudaMemcpyKind kind = p->memory == LBM_MEMORY_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    CUDA_CHECK(cudaMemcpyAsync(p->velocities, velDev, v3, kind, stream));
+    const cudaMemcpyKind back = p->memory == LBM_MEMORY_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
+    CUDA_CHECK(cudaMemcpyAsync(p->velocities, velDev, v3, back, stream));
     CUDA_CHECK(cudaMemcpyAsync(wallMomentum, dev->reflectWall, sizeof(double)*3, cudaMemcpyDeviceToHost, stream));
     CUDA_CHECK(cudaStreamSynchronize(stream));
 }
@@ -1187,7 +1211,7 @@ static void launchStencil(const void* A, const FluidView& f, const CouplingView&
     typedef typename Vec4<R>::type V;
     long long total = (long long) c.np*c.slots;
     int grid = (int) std::max(1LL, std::min(4736LL, (total + kThreads - 1)/kThreads));
-    stencilAxesKernel<<<std::max(1, (c.np + kThreads - 1)/kThreads), kThreads, 0, s>>>(c, pos, axisIndex, axisWeight,
+    stencilAxesKernel<<<std::max(1, std::min(4736, (c.np + kThreads/16 - 1)/(kThreads/16))), kThreads, 0, s>>>(c, pos, axisIndex, axisWeight,
                                                                                       firstIndex);
     // The stencil widths: 1 (nearest node), 2 (trilinear), 3 (three-point), 4 (Keys).
     auto claim = [&](auto w) {
@@ -1250,7 +1274,7 @@ void CouplingEngine::coupleWith(long long step, bool isStep, const CouplingView*
     const R* sw = (const R*) dev->slotWeight;
     const typename Vec4<R>::type* su = (const typename Vec4<R>::type*) dev->slotU;
     if (!centred) {
-        explicitKernel<R><<<warpGrid(np), kThreads, 0, stream>>>(f, c, velDev, dev->slotNode, sw, su, step, isStep,
+        explicitKernel<R><<<warpGrid(np), kThreads, 0, stream>>>(f, c, velIn, dev->slotNode, sw, su, step, isStep,
                                                                  forceOutDev, reaction, mask, wallDev);
         CUDA_CHECK(cudaGetLastError());
         fluid.launches++;
@@ -1267,7 +1291,7 @@ void CouplingEngine::coupleWith(long long step, bool isStep, const CouplingView*
             bits++;
         int cur = radixSortByKey(dev->keys, dev->values, dev->hist, np, bits, stream);
         fluid.launches += 3*((bits + 7)/8);
-        centeredNearestKernel<R><<<gridP, kThreads, 0, stream>>>(f, c, dev->keys[cur], dev->values[cur], velDev, forceInDev,
+        centeredNearestKernel<R><<<gridP, kThreads, 0, stream>>>(f, c, dev->keys[cur], dev->values[cur], velIn, forceIn,
                                                                   su, step, isStep, forceOutDev, reaction, mask, wallDev);
         CUDA_CHECK(cudaGetLastError());
         fluid.launches++;
@@ -1289,8 +1313,8 @@ void CouplingEngine::coupleWith(long long step, bool isStep, const CouplingView*
     R* coef = (R*) dev->coef;
     double* fout = forceOutDev;
     double* wall = wallDev;
-    double* fin = forceInDev;
-    double* vel = velDev;
+    const double* fin = forceIn;
+    const double* vel = velIn;
     int* sn = dev->slotNode;
     FluidView fv = f;
     CouplingView cc = c;
@@ -1304,8 +1328,9 @@ void CouplingEngine::coupleWith(long long step, bool isStep, const CouplingView*
         CUDA_CHECK(cudaLaunchCooperativeKernel((const void*) centeredSparseKernel<R>, dev->sparseGrid, kSolveThreads,
                                                sparseArgs, 0, stream));
         fluid.launches++;
-        CUDA_CHECK(cudaMemcpyAsync(status, statusDev, sizeof(int)*3, cudaMemcpyDeviceToHost, stream));
+        CUDA_CHECK(cudaMemcpyAsync(statusHost, statusDev, sizeof(int)*3, cudaMemcpyDeviceToHost, stream));
         CUDA_CHECK(cudaStreamSynchronize(stream));
+        std::memcpy(status, statusHost, sizeof(status));
     }
     if (spreadOnly || status[2] != 0) {
         launchSlotMomentsNow();
@@ -1416,6 +1441,10 @@ void CouplingEngine::prepare(const LbmParticleArrays* p, long long step, bool re
     preparedRemove = remove;
 }
 
+bool CouplingEngine::preparedFor(long long step, bool remove) const {
+    return prepared && step == preparedStep && remove == preparedRemove;
+}
+
 void CouplingEngine::joinPrepared() {
     if (prepared)
         CUDA_CHECK(cudaStreamWaitEvent(stream, ready, 0));
@@ -1429,7 +1458,7 @@ void CouplingEngine::discardPrepared() {
 void CouplingEngine::couple(long long step, bool isStep, bool remove) {
     const FluidView& f = fluid.deviceView();
     CouplingView c = makeCouplingView(lattice, f, np, widthOf(lattice.interpolation_stencil), massDev);
-    const bool usePrepared = prepared && isStep && step == preparedStep && remove == preparedRemove;
+    const bool usePrepared = isStep && preparedFor(step, remove);
     discardPrepared();
     if (!usePrepared)
         launchStencilPass(c, remove, isStep, stream);

@@ -20,8 +20,11 @@ public:
                    const double* masses, cudaStream_t stream);
     ~CouplingEngine();
     void setParameters(const LbmLatticeParameters& lattice);
-    // Load the particle arrays of a call into the device buffers (copies for host arrays).
-    void load(const LbmParticleArrays* particles, bool withForces);
+    // Take the particle arrays of a call: copies for host arrays; device arrays are read in place by the call's kernels,
+    // but for the positions, which the stencil pass may read on its own stream (not needed when it was prepared).
+    void load(const LbmParticleArrays* particles, bool withForces, bool withPositions = true);
+    // Whether the stencil pass of this step was prepared at beginStep.
+    bool preparedFor(long long step, bool remove) const;
     // Reflection at the walls (beginStep, ReferenceLBMKernels.cpp:315-338): reverses velocities on the device and
     // returns the momentum given to the wall, Da nm/ps (synchronizes).  The velocities are stored back.
     void reflect(const LbmParticleArrays* particles, double wallMomentum[3]);
@@ -76,7 +79,9 @@ private:
     double *posDev, *velDev, *forceInDev, *forceOutDev, *massDev;
     double* wallDev;           // 3 doubles: momentum of reactions on solid nodes
     int* statusDev;            // device status word of the conjugate gradients
+    const double *velIn = nullptr, *forceIn = nullptr;   // velocities and other forces of the call (load)
     double* pinned;            // pinned staging for host particle arrays
+    int* statusHost = nullptr; // behind it: the status words of a solve
     Device* dev;               // slot, sort and solver buffers
     int stencilSlots;
     int cgMaxIterations = kDefaultCgIterations;

@@ -131,32 +131,6 @@ __device__ double stencilKernel1(int stencil, double r) {
     }
 }
 
-// LBMStencils::axisWeights (LBMStencils.h:73-95): the nodes of the stencil along one axis and their weights,
-// clamped at open faces, with repeated nodes merged into their first slot.
-__device__ void axisWeights(int stencil, int width, double s, int n, bool open, int* index, double* weight) {
-    int first;
-    if (stencil == LBM_STENCIL_THREEPOINT)
-        first = (int) floor(s + 0.5) - 1;
-    else if (stencil == LBM_STENCIL_KEYS)
-        first = (int) floor(s) - 1;
-    else if (stencil == LBM_STENCIL_TRILINEAR)
-        first = (int) floor(s);
-    else
-        first = (int) floor(s + 0.5);
-    for (int i = 0; i < width; i++) {
-        weight[i] = stencilKernel1(stencil, s - (first + i));
-        int idx = first + i;
-        index[i] = open ? min(max(idx, 0), n - 1) : ((idx%n) + n)%n;
-    }
-    for (int i = 1; i < width; i++)
-        for (int j = 0; j < i; j++)
-            if (index[j] == index[i]) {
-                weight[j] += weight[i];
-                weight[i] = 0.0;
-                break;
-            }
-}
-
 // Density deviation and momentum of the post-stream populations of a node (pulled from the input array).
 template <typename T>
 __device__ void pullMomentsAt(const T* A, const FluidView& f, int x, int y, int z, double& dr, double& jx, double& jy,
@@ -185,43 +159,18 @@ __device__ void pullMoments(const T* A, const FluidView& f, long long node, doub
     pullMomentsAt<T>(A, f, (int) (node%f.nx), (int) (r%f.ny), (int) (r/f.ny), dr, jx, jy, jz);
 }
 
-// The node indices and weights of particle i's stencil on each axis (entries past the width: index -1, weight 0).
-__device__ __forceinline__ void stencilAxes(const CouplingView& c, const double* __restrict__ pos, int i, int index[3][4],
-                                            double weight[3][4]) {
-    const int size[3] = {c.nx, c.ny, c.nz};
-    for (int a = 0; a < 3; a++) {
-        for (int k = 0; k < 4; k++) {
-            index[a][k] = -1;
-            weight[a][k] = 0.0;
-        }
-        double sc = latticeCoordinate(pos[3*i+a], c.dx, size[a]);
-        if (c.stencil == LBM_STENCIL_NEAREST) {
-            // nearestNode (ReferenceLBMKernels.cpp:973-983): periodic wrap on every axis.
-            index[a][0] = ((int) floor(sc + 0.5))%size[a];
-            weight[a][0] = 1.0;
-        }
-        else
-            axisWeights(c.stencil, c.width, sc, size[a], c.open[a] != 0, index[a], weight[a]);
-    }
-}
-
-// The stencil slots t = i*slots + s of particle i by one warp: the node and weight of each slot (LBMStencils::axisWeights,
-// LBMStencils.h:73-95) and u = j/rho of the node pulled from the populations (after the momentum removal, :539, :672; a
-// solid node has rho = 0).  Lane 4 a + k < 12 forms entry k of axis a (index and weight, with axisWeights' merging of
-// repeated nodes), and each slot's lane takes its three entries by shuffles: a thread per slot formed all its particle's
-// entries again, nine to twelve kernel values in double with their roots, for the three that it uses (47 us per step of
-// 10,530 beads with the three-point stencil).  COHERENT: the positions were written by the same launch (a persistent
-// kernel): they are read through L2.
-template <typename T, typename R, bool COHERENT = false>
-__device__ __forceinline__ void stencilParticle(const T* __restrict__ A, const FluidView& f, const CouplingView& c,
-                                                const double* __restrict__ pos, int i, int lane, int remove,
-                                                int* slotNode, R* slotWeight, typename Vec4<R>::type* slotU) {
-    const int axis = min(lane >> 2, 2), k = lane & 3;
+// Entry k = lane % 4 of axis lane/4 % 4 (the last group repeats axis 2) of particle i's stencil (LBMStencils::axisWeights,
+// LBMStencils.h:73-95: clamped at open faces, repeated nodes merged into their first entry); lanes 12 and on of a group of 16 hold nothing of use.  Entries past the width: a negative index, weight 0.
+// Called by a whole warp.  COHERENT: the positions were written by the same launch.
+template <bool COHERENT>
+__device__ __forceinline__ void stencilEntry(const CouplingView& c, const double* __restrict__ pos, int i, int lane, int& index,
+                                             double& weight) {
+    const int axis = min((lane >> 2) & 3, 2), k = lane & 3;
     const int size = axis == 0 ? c.nx : (axis == 1 ? c.ny : c.nz);
     const double x = COHERENT ? __ldcg(&pos[3*i+axis]) : pos[3*i+axis];
     const double s = latticeCoordinate(x, c.dx, size);
-    int index = -1 - k;
-    double weight = 0.0;
+    index = -1 - k;
+    weight = 0.0;
     if (c.stencil == LBM_STENCIL_NEAREST) {
         if (k == 0) {
             index = ((int) floor(s + 0.5))%size;
@@ -233,11 +182,13 @@ __device__ __forceinline__ void stencilParticle(const T* __restrict__ A, const F
                         : (int) floor(s) - (c.stencil == LBM_STENCIL_KEYS ? 1 : 0);
         weight = stencilKernel1(c.stencil, s - (first + k));
         const int idx = first + k;
-        index = c.open[axis] ? min(max(idx, 0), size - 1) : ((idx%size) + size)%size;
+        const bool open = axis == 0 ? c.open[0] : (axis == 1 ? c.open[1] : c.open[2]);
+        index = open ? min(max(idx, 0), size - 1) : ((idx%size) + size)%size;
     }
     // A node that the axis meets more than once keeps the sum of its weights in its first entry.
     double merged = weight;
     bool repeated = false;
+#pragma unroll
     for (int j = 0; j < 4; j++) {
         const int other = __shfl_sync(0xffffffffu, index, (lane & ~3) + j);
         const double w = __shfl_sync(0xffffffffu, weight, (lane & ~3) + j);
@@ -247,6 +198,21 @@ __device__ __forceinline__ void stencilParticle(const T* __restrict__ A, const F
             merged += w;
     }
     weight = repeated ? 0.0 : merged;
+}
+
+// The stencil slots t = i*slots + s of particle i by one warp: the node and weight of each slot (LBMStencils::axisWeights,
+// LBMStencils.h:73-95) and u = j/rho of the node pulled from the populations (after the momentum removal, :539, :672; a
+// solid node has rho = 0).  Lane 4 a + k < 12 forms entry k of axis a (stencilEntry), and each slot's lane takes its three entries by shuffles: a thread per slot formed all its particle's
+// entries again, nine to twelve kernel values in double with their roots, for the three that it uses (47 us per step of
+// 10,530 beads with the three-point stencil).  COHERENT: the positions were written by the same launch (a persistent
+// kernel): they are read through L2.
+template <typename T, typename R, bool COHERENT = false>
+__device__ __forceinline__ void stencilParticle(const T* __restrict__ A, const FluidView& f, const CouplingView& c,
+                                                const double* __restrict__ pos, int i, int lane, int remove,
+                                                int* slotNode, R* slotWeight, typename Vec4<R>::type* slotU) {
+    int index;
+    double weight;
+    stencilEntry<COHERENT>(c, pos, i, lane, index, weight);
     const long long t0 = (long long) i*c.slots;
     for (int s0 = 0; s0 < c.slots; s0 += 32) {
         const int slot = s0 + lane, at = min(slot, c.slots - 1);

@@ -244,8 +244,12 @@ void B200Kernel::advanceFluid(const LbmParticleArrays* particles) {
     bool remove = lattice.momentum_removal_frequency > 0 && stepIndex%lattice.momentum_removal_frequency == 0;
     bool react = false;
     if (numParticles > 0) {
-        coupling->joinPrepared();
-        coupling->load(particles, lattice.drag_scheme == LBM_DRAG_CENTERED);
+        // Without prepared work to continue from, the positions are needed again, once the stream that may still read
+        // the last ones is done.
+        const bool ready = coupling->preparedFor(stepIndex, remove);
+        if (!ready)
+            coupling->joinPrepared();
+        coupling->load(particles, lattice.drag_scheme == LBM_DRAG_CENTERED, !ready);
         try {
             coupling->couple(stepIndex, true, remove);
         }
