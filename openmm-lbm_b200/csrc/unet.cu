@@ -189,15 +189,18 @@ __device__ __forceinline__ void drainStage(const Stage& st, int stage) {
 //
 // Warps 0-3 read the accumulators (bias, ReLU, BF16 stores), warp 4 issues the MMAs, warps 5-8 copy slices and
 // weight tiles with cp.async and hand them over through mbarriers.  The weights of one tap are a tile of
-// [8-channel group][output channel] x 16 bytes; all 27 stay resident when they fit (wSlots = 27), otherwise they
-// stream through a ring of wSlots tiles.
+// [8-channel group][output channel] x 16 bytes.  Where all 27 fit they stay resident, those of the three dz of a (dy, dx)
+// one below the other, and one MMA serves the three planes of a slice (their accumulators are neighbours, N = 3 nTile):
+// A is read once for three taps.  Otherwise they stream through a ring of wSlots tiles, a tap per MMA.
 //
 // Bound: an MMA of M = 128 and N <= 64 reads 4 KB of A (36 wavefronts of shared memory with 16 channels of B) and holds
-// the tensor core for 52 cycles, 41 us for 16 -> 16 channels on two 64 x 64 x 128 volumes.  Measured there: 47 us
-// (229 us with the gathering kernel, whose threads fetch every voxel 27 times and wait for each stage's MMAs); 48 -> 16
-// 124 us (880), 32 -> 32 at 32 x 32 x 64 30 us (84), 160 -> 160 at 8 x 8 x 16 38 us (307).  With one thread issuing from
-// divergent code the same layer took 82 us (its operands went through general registers, 140-200 cycles per MMA), and
-// with the planes' MMAs interleaved tap by tap 111 us (a branch per MMA).
+// the tensor core for 52 cycles: 41 us for 16 -> 16 channels on two 64 x 64 x 128 volumes with an MMA per tap, 15 us with
+// one for three.  Measured there: 40 us, 47 us with an MMA per tap (the copies of the slices, 1.4 times the volume in
+// pieces of 16 bytes, are what remains), 229 us with the gathering kernel, whose threads fetch every voxel 27 times and
+// wait for each stage's MMAs; 48 -> 16 channels 89 us (124, 880), 32 -> 32 at 32 x 32 x 64 20 us (30, 84), 160 -> 160 at
+// 8 x 8 x 16, streamed, 34 us (38, 307).  With one thread issuing from divergent code 16 -> 16 took 82 us (its operands
+// went through general registers, 140-200 cycles per MMA), and with the planes' MMAs interleaved tap by tap 111 us (a
+// branch per MMA).
 // ---------------------------------------------------------------------------------------------------------------
 
 constexpr int kTileX = 8, kTileY = 16, kHaloX = kTileX + 2, kHaloY = kTileY + 2;
@@ -224,13 +227,15 @@ struct SliceBarriers {
 };
 
 __host__ __device__ inline int sliceBytes(int cin) { return (cin/8)*kPlane; }
-// A weight tile: nTile channels of a group at 16 bytes, + 16 per group to spread the groups over the banks.
-__host__ __device__ inline int weightGroupBytes(int nTile) { return nTile*16 + 16; }
-__host__ __device__ inline int weightTileBytes(int cin, int nTile) { return (cin/8)*weightGroupBytes(nTile); }
+// A weight tile of `rows` rows: each group's at 16 bytes, + 16 per group to spread the groups over the banks.
+__host__ __device__ inline int weightGroupBytes(int rows) { return rows*16 + 16; }
+__host__ __device__ inline int weightTileBytes(int cin, int rows) { return (cin/8)*weightGroupBytes(rows); }
 __host__ __device__ inline size_t sliceSmemBytes(int cin, int nTile, int slots, int wSlots) {
     // The single-group layout pairs taps: a 28th tile of zeros and a zero slice stand in for the tap after the last.
-    return sizeof(SliceBarriers) + 128 + (size_t) slots*sliceBytes(cin) + (size_t) wSlots*weightTileBytes(cin, nTile)
-         + (cin == 8 ? kZeroZone + weightTileBytes(cin, nTile) : 0);
+    // Resident weights are 9 tiles of the three dz; streamed ones wSlots tiles of a tap.
+    const size_t weights = cin == 8 ? (size_t) (kTaps + 1)*weightTileBytes(cin, nTile) + kZeroZone
+                         : wSlots == kTaps ? (size_t) 9*weightTileBytes(cin, 3*nTile) : (size_t) wSlots*weightTileBytes(cin, nTile);
+    return sizeof(SliceBarriers) + 128 + (size_t) slots*sliceBytes(cin) + weights;
 }
 
 struct SliceItem {
@@ -242,14 +247,13 @@ __device__ __forceinline__ SliceItem sliceItem(const SliceParams& p, int item) {
     int r = item;
     const int cx = r%p.colsX; r /= p.colsX;
     const int cy = r%p.colsY; r /= p.colsY;
-    const int zb = r%p.zBlocks; r /= p.zBlocks;
-    const int nb = r%p.nBlocks;
-    t.n = r/p.nBlocks;
+    const int zb = r%p.zBlocks;
+    t.n = r/p.zBlocks;
     t.x0 = cx*kTileX;
     t.y0 = cy*kTileY;
     t.z0 = zb*p.zLen;
     t.zc = min(p.zLen, p.D - t.z0);
-    t.co0 = nb*p.nTile;
+    t.co0 = blockIdx.y*p.nTile;
     return t;
 }
 
@@ -367,7 +371,9 @@ __global__ void __launch_bounds__(sliceThreads<MODE>)
 convSliceKernel(const SliceParams p) {
     extern __shared__ __align__(128) uint8_t smemRaw[];
     SliceBarriers* bars = reinterpret_cast<SliceBarriers*>(smemRaw);
-    const int slotBytes = sliceBytes(p.cin), tileBytes = weightTileBytes(p.cin, p.nTile);
+    // Rows of a weight tile: a tap's output channels, or those of the three dz of a (dy, dx), dz = 2 first.
+    const int tileRows = MODE == kResident ? 3*p.nTile : p.nTile;
+    const int slotBytes = sliceBytes(p.cin), tileBytes = weightTileBytes(p.cin, tileRows);
     const uint32_t ring = (smemAddr(smemRaw) + (uint32_t) sizeof(SliceBarriers) + 127u) & ~127u;
     const uint32_t zeroZone = ring + (uint32_t) (p.slots*slotBytes);
     const uint32_t weights = zeroZone + (p.cin == 8 ? kZeroZone : 0);
@@ -389,7 +395,7 @@ convSliceKernel(const SliceParams p) {
             init(&bars->empty[i], 1);
         }
         for (int i = 0; i < p.wSlots; i++) {
-            init(&bars->wFull[i], resident ? producerThreads : 32);
+            init(&bars->wFull[i], producerThreads);
             init(&bars->wEmpty[i], 1);
         }
         for (int i = 0; i < p.accSlots; i++) {
@@ -415,19 +421,17 @@ convSliceKernel(const SliceParams p) {
     const int groups = p.cin/8;
 
     if (warp >= 5) {
-        // ---- producers: slices in the order of the planes (all warps share a slice), and the weight tiles in the order
-        // of their use (one warp each in turn when streamed, so that the tiles' latencies overlap) ----
+        // ---- producers: slices in the order of the planes and the weight tiles in the order of their use, each shared by
+        // all threads (a streamed tile by one warp: 224 -> 64 channels at 16x16x32 x 2 in 74 us instead of 59) ----
         const int t = tid - (kEpilogueThreads + 32), producers = producerThreads;
-        // At most wSlots warps: one that is further ahead would take a slot's phase for the one two before it.
-        const int pw = warp - 5, warps = min(producers/32, p.wSlots);
         CopyQueue queue;
-        const Pieces bySlice(t, producers, groups), byTile(lane, 32, groups), byAll(t, producers, groups);
-        const int groupW = weightGroupBytes(p.nTile);
-        int tile = 0, slot = 0, wSlot = 0;
+        const Pieces bySlice(t, producers, groups), byAll(t, producers, groups);
+        const int groupW = weightGroupBytes(tileRows);
+        int slot = 0, wSlot = 0;
         uint32_t slotPhase = 1, wPhase = 1;        // a free slot's barrier has completed the phase before its first
         bool ok = true;
-        auto copyTile = [&](const Pieces& pieces, int at, int tap, int co0) {
-            const uint32_t base = weights + (uint32_t) (at*tileBytes);
+        auto copyTile = [&](const Pieces& pieces, int at, int row, int tap, int co0) {
+            const uint32_t base = weights + (uint32_t) (at*tileBytes + row*16);
             const __nv_bfloat16* src = p.w + ((size_t) co0*kTaps + tap)*p.cin;
             for (int g = pieces.g, n = pieces.v; n < p.nTile; ) {
                 copy16(base + (uint32_t) (g*groupW + n*16), src + (size_t) n*kTaps*p.cin + 8*g, true);
@@ -462,16 +466,15 @@ convSliceKernel(const SliceParams p) {
                         continue;
                     for (int k = 0; k < 9 && ok; k++) {
                         if (resident) {
-                            copyTile(byAll, 9*dz + k, 9*dz + k, it.co0);
+                            MODE == kResident ? copyTile(byAll, k, (2 - dz)*p.nTile, 9*dz + k, it.co0)
+                                              : copyTile(byAll, 9*dz + k, 0, 9*dz + k, it.co0);
                             continue;
                         }
-                        if (tile++%warps == pw) {
-                            ok = queue.waitFree(smemAddr(&bars->wEmpty[wSlot]), wPhase, limit, stop);
-                            if (!ok)
-                                break;
-                            copyTile(byTile, wSlot, 9*dz + k, it.co0);
-                            queue.push(smemAddr(&bars->wFull[wSlot]));
-                        }
+                        ok = queue.waitFree(smemAddr(&bars->wEmpty[wSlot]), wPhase, limit, stop);
+                        if (!ok)
+                            break;
+                        copyTile(byAll, wSlot, 0, 9*dz + k, it.co0);
+                        queue.push(smemAddr(&bars->wFull[wSlot]));
                         if (++wSlot == p.wSlots) {
                             wSlot = 0;
                             wPhase ^= 1;
@@ -488,8 +491,8 @@ convSliceKernel(const SliceParams p) {
         // ---- the MMAs: the instructions between two of them are what a narrow layer waits for, so the taps are
         // unrolled, a descriptor is its low word plus a constant, and the warp stays converged (uniform registers) ----
         {
-            const uint32_t idesc = instrDescriptor(p.nTile);
-            const uint32_t groupW = (uint32_t) weightGroupBytes(p.nTile), tileUnits = (uint32_t) tileBytes/16;
+            const uint32_t idesc = instrDescriptor(p.nTile), idesc2 = instrDescriptor(2*p.nTile), idesc3 = instrDescriptor(3*p.nTile);
+            const uint32_t groupW = (uint32_t) weightGroupBytes(tileRows), tileUnits = (uint32_t) tileBytes/16;
             const uint32_t aHigh = (kHaloX*16 >> 4) | (1u << 14), bHigh = (128 >> 4) | (1u << 14);
             const uint32_t wLow = (weights >> 4) | ((MODE == kSingleGroup ? (uint32_t) tileBytes : groupW) >> 4 << 16);
             int plane0 = 0, slot = 0, wSlot = 0;
@@ -502,6 +505,64 @@ convSliceKernel(const SliceParams p) {
                     if (!ok)
                         break;
                     const uint32_t base = ring + (uint32_t) (slot*slotBytes);
+                    if constexpr (MODE == kResident) {
+                        // The slice's planes s - 2, s - 1 and s take the taps dz = 2, 1 and 0 of every (dy, dx) from the
+                        // same rows of A: one MMA with their accumulators side by side (two where the ring of
+                        // accumulators wraps around between them).
+                        const int lo = max(0, s - 2), hi = min(it.zc - 1, s), count = hi - lo + 1;
+                        if (hi == s && plane0 + s >= p.accSlots) {
+                            const int plane = plane0 + s;
+                            ok = warpWait(smemAddr(&bars->accEmpty[plane%p.accSlots]), (uint32_t) ((plane/p.accSlots - 1) & 1), limit, stop);
+                            fenceAfterSync();
+                        }
+                        if (item == blockIdx.x && s <= 2)
+                            ok = ok && warpWait(smemAddr(&bars->wFull[s]), 0, limit, stop);
+                        if (!ok)
+                            break;
+                        issued = true;
+                        const uint32_t aLow = (base >> 4) | (uint32_t) (kPlane/16) << 16;
+                        // The MMAs of (dy, dx) = r for `n` planes from accumulator `acc` on, rows of the tile from `row` on.
+                        auto multiply = [&](int r, int acc, uint32_t row, int n, uint32_t accumulate) {
+                            const uint32_t d = tmem + (uint32_t) (acc*p.nTile), id = n == 3 ? idesc3 : (n == 2 ? idesc2 : idesc);
+                            uint32_t a = aLow + (uint32_t) ((r/3)*kHaloX + r%3), b = wLow + (uint32_t) r*tileUnits + row;
+                            mmaElected(d, join(a, aHigh), join(b, bHigh), id, accumulate);
+                            for (int g = 2; g < groups; g += 2) {
+                                a += 2*kPlane/16;
+                                b += groupW/8;
+                                mmaElected(d, join(a, aHigh), join(b, bHigh), id, 1u);
+                            }
+                        };
+                        const int acc = (plane0 + lo)%p.accSlots, head = min(count, p.accSlots - acc), tail = count - head;
+                        const uint32_t row = (uint32_t) ((2 - s + lo)*p.nTile), rowTail = row + (uint32_t) (head*p.nTile);
+                        // A plane that starts here overwrites its accumulator in its first MMA.
+                        if (hi == s) {
+                            const int older = count - 1, olderHead = min(older, head), olderTail = older - olderHead;
+                            if (olderHead > 0)
+                                multiply(0, acc, row, olderHead, 1u);
+                            if (olderTail > 0)
+                                multiply(0, 0, rowTail, olderTail, 1u);
+                            multiply(0, (plane0 + s)%p.accSlots, 2u*(uint32_t) p.nTile, 1, 0u);
+                        }
+                        else {
+                            multiply(0, acc, row, head, 1u);
+                            if (tail > 0)
+                                multiply(0, 0, rowTail, tail, 1u);
+                        }
+                        if (tail == 0) {
+#pragma unroll
+                            for (int r = 1; r < 9; r++)
+                                multiply(r, acc, row, head, 1u);
+                        }
+                        else {
+#pragma unroll
+                            for (int r = 1; r < 9; r++) {
+                                multiply(r, acc, row, head, 1u);
+                                multiply(r, 0, rowTail, tail, 1u);
+                            }
+                        }
+                        if (s >= 2)
+                            commitElected(smemAddr(&bars->accFull[(plane0 + s - 2)%p.accSlots]));
+                    }
                     auto stage = [&](auto dzc) {
                         constexpr int dz = decltype(dzc)::value;
                         const int k0 = s - dz;
@@ -565,9 +626,11 @@ convSliceKernel(const SliceParams p) {
                         if (dz == 2)
                             commitElected(smemAddr(&bars->accFull[acc]));
                     };
-                    stage(std::integral_constant<int, 2>());
-                    stage(std::integral_constant<int, 1>());
-                    stage(std::integral_constant<int, 0>());
+                    if constexpr (MODE != kResident) {
+                        stage(std::integral_constant<int, 2>());
+                        stage(std::integral_constant<int, 1>());
+                        stage(std::integral_constant<int, 0>());
+                    }
                     if (!ok)
                         break;
                     // The slice is free once its MMAs are done; with one group the next slice's first pair still reads
@@ -729,10 +792,10 @@ convForwardKernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __re
 // one) that are read and cleared while the next unit fills.
 //
 // Bound: 16 -> 16 channels read 4 KB of x and 4.6 KB of dy (68 wavefronts of shared memory) per MMA and 16 voxels, 19 us
-// on two 64 x 64 x 128 volumes.  Measured there: 90 us, what remains being the copies (dy three times) and the atomics of
-// the finished sums (65 us, with an error of 4e-6 instead of 9e-7, when a CTA adds its sums once); 1150 us with the
-// kernel before it, which gathered both operands transposed element by element and waited for each stage.  48 -> 16:
-// 180 us (4000), 32 -> 32 at 32 x 32 x 64 30 us (314), 160 -> 160 at 8 x 8 x 16 24 us (116).
+// on two 64 x 64 x 128 volumes.  Measured there: 79 us, what remains being the copies (dy three times) and the atomics of
+// the finished sums (a quarter less, with an error of 4e-6 instead of 9e-7, when a CTA adds its sums once); 1150 us with
+// the kernel before it, which gathered both operands transposed element by element and waited for each stage.  48 -> 16:
+// 160 us (4000), 32 -> 32 at 32 x 32 x 64 29 us (314), 160 -> 160 at 8 x 8 x 16 25 us (116).
 // ---------------------------------------------------------------------------------------------------------------
 
 constexpr int kRunX = 16, kRowsY = 8;
@@ -740,6 +803,8 @@ constexpr int kGroupPitch = kRunX*16 + 16;     // bytes of a group's 16 voxels; 
 constexpr int kGradSlots = 4;
 constexpr int kGradProducers = 256, kGradReaders = 256;
 constexpr int kGradThreads = kGradProducers + 32 + kGradReaders, kMaxUnits = 5;
+constexpr int kGradPiecesX = 4;                // (kRowsY + 2) kRunX 5 groups / kGradProducers
+constexpr int kGradPieces = 6;                 // up to 32 output channels; more are placed piece by piece
 
 struct GradParams {
     const __nv_bfloat16* x;
@@ -843,16 +908,66 @@ convSliceGradKernel(const GradParams p) {
         int slot = 0, buffer = 0;
         uint32_t slotPhase = 1, dyPhase = 1;         // a free slot's barrier has completed the phase before its first
         bool ok = true;
+        // A thread's pieces have the same place in a slice, or in a plane of dy, and the same distance in memory from the
+        // item's origin, for every item: both are formed once, an item adds which of them lie in the volume, and a copy is
+        // a few instructions (16 -> 16 channels on two 64 x 64 x 128 volumes: 78 us, 87 with them formed for every copy).
+        const int totalX = (kRowsY + 2)*kRunX*groupsX, totalY = kRowsY*3*kRunX*groupsY;
+        const int mineX = (totalX - tid + kGradProducers - 1)/kGradProducers;
+        const bool fewY = totalY <= kGradPieces*kGradProducers;
+        const int mineY = fewY ? (totalY - tid + kGradProducers - 1)/kGradProducers : 0;
+        uint32_t placeX[kGradPiecesX], placeY[kGradPieces], whereX[kGradPiecesX], whereY[kGradPieces];
+        ptrdiff_t fromX[kGradPiecesX], fromY[kGradPieces];
+        {
+            int g = byX.g, v = byX.v;
+#pragma unroll
+            for (int j = 0; j < kGradPiecesX; j++) {
+                const int k = v%kRunX, y = v/kRunX;
+                placeX[j] = (uint32_t) ((y*groupsX + g)*kGroupPitch + k*16);
+                fromX[j] = ((ptrdiff_t) (y - 1)*p.W + k)*p.cin + 8*g;
+                whereX[j] = (uint32_t) (y | k << 16);
+                byX.next(g, v);
+            }
+            g = byY.g;
+            v = byY.v;
+#pragma unroll
+            for (int j = 0; j < kGradPieces; j++) {
+                const int k = v%kRunX, r = v/kRunX, y = r/3, dx = r - 3*y;
+                placeY[j] = (uint32_t) (((y*p.zLen*3 + dx)*groupsY + g)*kGroupPitch + k*16);
+                fromY[j] = ((ptrdiff_t) y*p.W + k + 1 - dx)*p.cout + 8*g;
+                whereY[j] = (uint32_t) (y | (k + 2 - dx) << 16);
+                byY.next(g, v);
+            }
+        }
         for (int i = blockIdx.x; i < p.items && ok; i += gridDim.x) {
             int n, z0, zc, y0, x0;
             item(i, n, z0, zc, y0, x0);
+            const size_t origin = (size_t) y0*p.W + x0;
+            uint32_t inX = 0, inY = 0;
+#pragma unroll
+            for (int j = 0; j < kGradPiecesX; j++)
+                if ((unsigned) (y0 - 1 + (int) (whereX[j] & 0xFFFFu)) < (unsigned) p.H && x0 + (int) (whereX[j] >> 16) < p.W)
+                    inX |= 1u << j;
+#pragma unroll
+            for (int j = 0; j < kGradPieces; j++)
+                if (y0 + (int) (whereY[j] & 0xFFFFu) < p.H && (unsigned) (x0 - 1 + (int) (whereY[j] >> 16)) < (unsigned) p.W)
+                    inY |= 1u << j;
             ok = queue.waitFree(smemAddr(&bars->dyEmpty[buffer]), dyPhase, limit, stop);
             for (int j = 0; j < zc + halo && ok; j++) {
                 if (j < zc) {
                     // Plane z0 + j of dy: copy dx holds dy at x - (dx - 1).
                     const __nv_bfloat16* plane = p.dy + ((size_t) n*p.D + z0 + j)*p.H*p.W*p.cout + co0;
                     const uint32_t base = dyBase + (uint32_t) (buffer*dyBytes);
-                    for (int g = byY.g, v = byY.v; v < kRowsY*3*kRunX; ) {
+                    if (fewY) {
+                        const uint32_t at = base + (uint32_t) (j*3*groupsY*kGroupPitch);
+                        const __nv_bfloat16* from = plane + origin*p.cout;
+#pragma unroll
+                        for (int k = 0; k < kGradPieces; k++)
+                            if (k < mineY) {
+                                const bool valid = (inY >> k) & 1u;
+                                copy16(at + placeY[k], valid ? from + fromY[k] : p.dy, valid);
+                            }
+                    }
+                    else for (int g = byY.g, v = byY.v; v < kRowsY*3*kRunX; ) {
                         const int k = v%kRunX, r = v/kRunX, y = r/3, dx = r%3;
                         const int yy = y0 + y, xx = x0 + k + 1 - dx;
                         const bool valid = yy < p.H && (unsigned) xx < (unsigned) p.W;
@@ -868,13 +983,13 @@ convSliceGradKernel(const GradParams p) {
                 const bool inside = z >= 0 && z < p.D;
                 const __nv_bfloat16* plane = p.x + ((size_t) n*p.D + (inside ? z : 0))*p.H*p.W*p.cin + 8*group0;
                 const uint32_t base = ring + (uint32_t) (slot*slotBytes);
-                for (int g = byX.g, v = byX.v; v < (kRowsY + 2)*kRunX; ) {
-                    const int k = v%kRunX, y = v/kRunX, yy = y0 + y - 1, xx = x0 + k;
-                    const bool valid = inside && (unsigned) yy < (unsigned) p.H && xx < p.W;
-                    copy16(base + (uint32_t) ((y*groupsX + g)*kGroupPitch + k*16),
-                           plane + (valid ? ((size_t) yy*p.W + xx)*p.cin + 8*g : 0), valid);
-                    byX.next(g, v);
-                }
+                const __nv_bfloat16* from = plane + origin*p.cin;
+#pragma unroll
+                for (int k = 0; k < kGradPiecesX; k++)
+                    if (k < mineX) {
+                        const bool valid = inside && ((inX >> k) & 1u);
+                        copy16(base + placeX[k], valid ? from + fromX[k] : p.x, valid);
+                    }
                 queue.push(smemAddr(&bars->full[slot]));
                 if (++slot == kGradSlots) {
                     slot = 0;
@@ -912,14 +1027,22 @@ convSliceGradKernel(const GradParams p) {
                 const int first = max(0, j - halo), last = min(zc - 1, j);
                 const int count = last - first + 1, step = merged ? count : 1;
                 const uint32_t idesc = instrDescriptor(step*width) | (1u << 15) | (1u << 16);
-                uint32_t a = low | ((ring + (uint32_t) (slot*slotBytes)) >> 4);
-                uint32_t b = low | (((dyBase + (uint32_t) (buffer*dyBytes)) >> 4) + (uint32_t) first*planeY);
-                for (int y = 0; y < rows; y++, a += rowX, b += rowY)
-                    for (int k = 0; k < count; k += step) {
-                        const int column = halo - j + first + k, at = unit + column;
-                        mmaElected(tmem + (uint32_t) (merged ? unit*unitWidth + column*width : (at >= units ? at - units : at)*width),
-                                   join(a, high), join(b + (uint32_t) k*planeY, high), idesc, 1u);
+                const uint32_t a = low | ((ring + (uint32_t) (slot*slotBytes)) >> 4);
+                const uint32_t b = low | (((dyBase + (uint32_t) (buffer*dyBytes)) >> 4) + (uint32_t) first*planeY);
+                // The rows of an accumulator one after another: an MMA is two additions and its issue (90 -> 87 us).
+                for (int k = 0; k < count; k += step) {
+                    const int column = halo - j + first + k, at = unit + column;
+                    const uint32_t d = tmem + (uint32_t) (merged ? unit*unitWidth + column*width : (at >= units ? at - units : at)*width);
+                    const uint32_t bk = b + (uint32_t) k*planeY;
+                    if (rows == kRowsY) {
+#pragma unroll
+                        for (int y = 0; y < kRowsY; y++)
+                            mmaElected(d, join(a + (uint32_t) y*rowX, high), join(bk + (uint32_t) y*rowY, high), idesc, 1u);
                     }
+                    else
+                        for (int y = 0; y < rows; y++)
+                            mmaElected(d, join(a + (uint32_t) y*rowX, high), join(bk + (uint32_t) y*rowY, high), idesc, 1u);
+                }
                 issued = true;
                 commitElected(smemAddr(&bars->empty[slot]));
                 if (++slot == kGradSlots) {
@@ -1007,9 +1130,9 @@ size_t stageBytes(int rowsB) {
 // (cin of an odd number of 8-channel groups other than one, whose 16-channel steps straddle taps; slices too wide for
 // two slots in shared memory, above 224-240 channels): the gathering kernel takes those.  Where both apply the slices
 // are faster from the smallest volumes on (one voxel, 16 -> 16: 8 against 15 us).
-constexpr size_t kSmemLimit = 227*1024, kSmemHalf = 113*1024, kSmemQuarter = 56*1024;
+constexpr size_t kSmemLimit = 227*1024, kSmemHalf = 113*1024;
 
-bool planSlices(SliceParams& p, int sms, size_t& smem, int& grid) {
+bool planSlices(SliceParams& p, int sms, size_t& smem, dim3& grid) {
     if (p.cin != 8 && p.cin%16 != 0)
         return false;
     p.colsX = (p.W + kTileX - 1)/kTileX;
@@ -1017,61 +1140,83 @@ bool planSlices(SliceParams& p, int sms, size_t& smem, int& grid) {
     const long long columns = (long long) p.colsX*p.colsY*p.batch;
     if (columns*p.D > (1LL << 28) || (long long) p.H*p.W*p.cin >= (1LL << 31))
         return false;
-    // Output channels per CTA: at most 112 (four accumulators in tensor memory), those with the least time by the MMAs
-    // alone, rounds of items times the cycles of an MMA (32 for up to 64 channels, its reading of A; then N/2): wide
-    // tiles read A less often, narrow ones spread few planes over more SMs.
-    long long best = -1;
+    // The output channels and planes per item and the place of the weights, by an estimate of the time in cycles: the
+    // rounds of items over the SMs times the slower of an item's MMAs and its copies, and the copies before the first
+    // MMA.  An MMA of 16 channels takes the 52 cycles that were measured for N = 16, more as N grows (36 + N/4 wavefronts
+    // of shared memory, N/2 of the tensor core); an SM copies about 40 bytes per cycle from L2; a streamed tile of weights
+    // takes 1000 cycles to be handed over and 1 per 15 bytes.
+    const double kCopy = 40.0, kStream = 15.0, kTile = 1000.0;
+    const int steps = (p.cin + 15)/16;
+    auto mma = [](int n) { return std::max(52.0, std::max(44.0 + n/4.0, 10.0 + n/2.0)); };
+    double best = 0;
+    bool found = false;
     for (int n = std::min(112, p.cout); n >= 16; n -= 16) {
         if (p.cout%n != 0)
             continue;
-        const long long cost = (columns*p.D*(p.cout/n) + sms - 1)/sms*std::max(32, n/2);
-        if (best < 0 || cost < best) {
-            best = cost;
-            p.nTile = n;
+        for (int zLen = 8; zLen >= 1; zLen /= 2) {
+            if (zLen > 1 && (zLen/2 >= p.D || (p.cin == 8 && p.D%zLen != 0)))
+                continue;
+            SliceParams t = p;
+            t.nTile = n;
+            t.nBlocks = p.cout/n;
+            t.zLen = zLen;
+            t.zBlocks = (p.D + zLen - 1)/zLen;
+            const long long items = columns*t.zBlocks;
+            const double rounds = items*t.nBlocks < 4LL*sms ? (double) ((items*t.nBlocks + sms - 1)/sms)
+                                                            : (double) (items*t.nBlocks)/sms;
+            const double slices = (zLen + 2)*(double) kSliceVoxels*p.cin*2, weights = (double) kTaps*p.cin*n*2;
+            auto consider = [&](int slots, int wSlots, double work, double copies, double before) {
+                if (sliceSmemBytes(p.cin, n, slots, wSlots) > kSmemLimit)
+                    return false;
+                const double cost = rounds*std::max(work, copies/kCopy) + before/kCopy;
+                if (!found || cost < best) {
+                    best = cost;
+                    found = true;
+                    t.slots = slots;
+                    t.wSlots = wSlots;
+                    // Accumulators: three in progress and one being read, more where they cost no CTA its place, so that
+                    // their ring seldom wraps around between the planes of a slice.
+                    const bool two = sliceSmemBytes(p.cin, n, slots, wSlots) <= kSmemHalf && n <= 64;
+                    t.accSlots = p.cin == 8 || wSlots < kTaps ? (n < 32 ? kMaxAcc : 4) : std::min(kMaxAcc, (two ? 256 : 512)/n);
+                    t.items = (int) items;
+                    p = t;
+                }
+                return true;
+            };
+            const double slice = slices/(zLen + 2);
+            if (p.cin == 8)
+                // The slots of an item are consecutive (a pair of taps spans two slices): two items' worth of them.
+                consider(2*(zLen + 2), kTaps, 14.0*zLen*mma(n), slices, weights + 3*slice);
+            else {
+                const int threes = std::max(0, zLen - 2);
+                const double merged = 9.0*steps*(2*mma(n) + (zLen > 1 ? 2*mma(2*n) : mma(n)) + threes*mma(3*n));
+                bool resident = false;
+                for (int slots = 6; slots >= 3 && n <= 80 && !resident; slots--)
+                    if (slots == 3 || sliceSmemBytes(p.cin, n, slots, kTaps) <= kSmemHalf)
+                        resident = consider(slots, kTaps, merged, slices, weights + slice);
+                const double streamed = zLen*(weights/kStream + kTaps*kTile);
+                for (int tiles = 12; tiles >= 2; tiles--)
+                    if ((zLen > 1 && consider(3, tiles, 27.0*steps*zLen*mma(n), slices + streamed*kCopy, slice)) ||
+                        consider(2, tiles, 27.0*steps*zLen*mma(n), slices + streamed*kCopy, slice))
+                        break;
+            }
         }
-    }
-    p.nBlocks = p.cout/p.nTile;
-    p.accSlots = p.nTile < 32 ? kMaxAcc : 4;
-    // Planes per item: long runs load fewer slices twice, short ones balance the SMs.
-    p.zLen = 8;
-    while (p.zLen > 1 && (columns*((p.D + p.zLen - 1)/p.zLen)*p.nBlocks < 3*sms || (p.cin == 8 && p.D%p.zLen != 0)))
-        p.zLen /= 2;
-    p.zBlocks = (p.D + p.zLen - 1)/p.zLen;
-    const long long items = columns*p.zBlocks*p.nBlocks;
-    p.items = (int) items;
-    // Slots, with all weights resident if they fit beside at least three slices (two CTAs per SM if those fit), else
-    // with a ring of weight tiles.  A CTA of several items keeps its weights only if all items have the same channels.
-    const bool keep = p.nBlocks == 1 || items <= sms;
-    auto fits = [&](int slots, int wSlots, size_t limit) {
-        if (sliceSmemBytes(p.cin, p.nTile, slots, wSlots) > limit)
-            return false;
-        p.slots = slots;
-        p.wSlots = wSlots;
-        return true;
-    };
-    bool found = false;
-    if (p.cin == 8) {
-        // The slots of an item are consecutive (a pair of taps spans two slices): two items' worth of them.
-        found = keep && fits(2*(p.zLen + 2), kTaps, kSmemLimit);
-    }
-    else {
-        for (size_t limit : {kSmemQuarter, kSmemHalf, kSmemLimit})
-            for (int slots = 6; slots >= 3 && keep && !found; slots--)
-                found = fits(slots, kTaps, limit);
-        for (int n = 8; n >= 4 && !found && items > sms; n--)
-            found = fits(3, n, kSmemHalf);
-        for (int n = 12; n >= 2 && !found; n--)
-            found = (p.zLen > 1 && fits(3, n, kSmemLimit)) || fits(2, n, kSmemLimit);
     }
     if (!found)
         return false;
+    // More slots where they cost no CTA its place.
+    if (p.cin != 8 && p.wSlots == kTaps)
+        while (p.slots < 6 && sliceSmemBytes(p.cin, p.nTile, p.slots + 1, kTaps) <= kSmemLimit &&
+               (sliceSmemBytes(p.cin, p.nTile, p.slots, kTaps) > kSmemHalf ||
+                sliceSmemBytes(p.cin, p.nTile, p.slots + 1, kTaps) <= kSmemHalf))
+            p.slots++;
     smem = sliceSmemBytes(p.cin, p.nTile, p.slots, p.wSlots);
     // Several CTAs per SM where shared and tensor memory allow: one thread issues a CTA's MMAs and is slower than the
     // tensor core on narrow layers.
     int perSM = 1;
     while (perSM < 4 && (smem + 1024)*(perSM + 1) <= kSmemLimit + 1024 && tmemColumns(p.accSlots*p.nTile)*(perSM + 1) <= 512)
         perSM++;
-    grid = (int) std::min(items, (long long) perSM*sms);
+    grid = dim3((unsigned) std::max(1, std::min(p.items, perSM*sms/p.nBlocks)), (unsigned) p.nBlocks);
     return true;
 }
 
@@ -1134,7 +1279,8 @@ LbmStatus lbm_conv3d_forward(const void* x, const void* w, const float* bias, vo
     p.bias = bias;
     p.y = (__nv_bfloat16*) y;
     p.batch = batch; p.D = depth; p.H = height; p.W = width; p.cin = cin; p.cout = cout; p.relu = relu;
-    int device = 0, sms = 148, grid = 0;
+    int device = 0, sms = 148;
+    dim3 grid;
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     size_t smem = 0;
