@@ -44,6 +44,8 @@ LbmStatus lbm_conv3d_set_wait_limit(long long polls);
  *   upsample_concat  y = the nearest 2x upsampling of x, then skip, along the channels (even sizes), and its gradients
  *   relu_bias_grad   out = dy where y > 0 and 0 dy elsewhere, db[channels] += its sums over the voxels (FP32); with y NULL
  *                    the sums of dy alone
+ *   weights          of every layer the FP32 weights w[cout][27][cin] in BF16, and where wt[layer] is not NULL flipped and
+ *                    transposed, wt[cin][26 - tap][cout]; the tables are host memory, no alignment is asked for
  *   input            the network's input for one solid mask (bytes): mask, inlet, xs[x], ys[y], zs[z] and three zeros per
  *                    voxel */
 LbmStatus lbm_net_pool(const void* x, void* y, int batch, int depth, int height, int width, int channels, void* stream);
@@ -55,6 +57,8 @@ LbmStatus lbm_net_upsample_concat_grad(const void* dy, void* dx, void* dskip, in
                                        int channels, int skip_channels, void* stream);
 LbmStatus lbm_net_relu_bias_grad(const void* dy, const void* y, void* out, float* db, long long voxels, int channels,
                                  void* stream);
+LbmStatus lbm_net_weights(int layers, const float* const* w, void* const* w16, void* const* wt, const int* cout,
+                          const int* cin, void* stream);
 LbmStatus lbm_net_input(const void* mask, float inlet, const float* xs, const float* ys, const float* zs, void* out,
                         int depth, int height, int width, void* stream);
 

@@ -183,6 +183,53 @@ inputKernel(const unsigned char* __restrict__ mask, float inlet, const float* __
     }
 }
 
+// The convolutions' weights as they read them: w16 the FP32 weights [cout][27][cin] in BF16, wt (where asked for) the
+// flipped, transposed ones [cin][26 - tap][cout] of the input gradient.  A block takes 32 x 32 weights of a tap; the
+// layers of a launch come in a table in its parameters.  Bound by launches, not by its bytes: the 15 layers of the network
+// are one launch of 6 us, 9 us with the transposed ones (a cast per layer, and for the gradient a flip and a copy, were
+// 43 launches and 180 us of the device, and 6 us each of the host).
+constexpr int kLayers = 32, kTile = 32;
+struct WeightTable {
+    const float* w[kLayers];
+    __nv_bfloat16* w16[kLayers];
+    __nv_bfloat16* wt[kLayers];
+    int cout[kLayers], cin[kLayers];
+    unsigned first[kLayers + 1];       // blocks of the layers before
+};
+
+__global__ void __launch_bounds__(kThreads) weightsKernel(const __grid_constant__ WeightTable t) {
+    __shared__ __nv_bfloat16 tile[kTile][kTile + 2];
+    int layer = 0;
+    while (blockIdx.x >= t.first[layer + 1])
+        layer++;
+    const int cout = t.cout[layer], cin = t.cin[layer], tilesI = (cin + kTile - 1)/kTile;
+    unsigned r = blockIdx.x - t.first[layer];
+    const int tap = (int) (r%27u);
+    r /= 27u;
+    const int i0 = (int) (r%(unsigned) tilesI)*kTile, o0 = (int) (r/(unsigned) tilesI)*kTile;
+    const int lane = threadIdx.x%kTile, row = threadIdx.x/kTile;
+    const float* w = t.w[layer];
+    __nv_bfloat16 *w16 = t.w16[layer], *wt = t.wt[layer];
+    constexpr int kRows = kThreads/kTile, kEach = kTile/kRows;
+    const size_t at = ((size_t) (o0 + row)*27 + tap)*cin + i0 + lane, step = (size_t) kRows*27*cin;
+    float v[kEach];
+#pragma unroll
+    for (int k = 0; k < kEach; k++)
+        v[k] = o0 + row + k*kRows < cout && i0 + lane < cin ? __ldg(w + at + k*step) : 0.0f;
+#pragma unroll
+    for (int k = 0; k < kEach; k++)
+        if (o0 + row + k*kRows < cout && i0 + lane < cin) {
+            tile[row + k*kRows][lane] = __float2bfloat16_rn(v[k]);
+            w16[at + k*step] = tile[row + k*kRows][lane];
+        }
+    if (wt == nullptr)
+        return;
+    __syncthreads();
+    for (int i = row; i < kTile; i += kRows)
+        if (i0 + i < cin && o0 + lane < cout)
+            wt[((size_t) (i0 + i)*27 + 26 - tap)*cout + o0 + lane] = tile[lane][i];
+}
+
 LbmStatus invalid(const char* message) {
     lbm::setLastError(message);
     return LBM_ERR_INVALID_ARGUMENT;
@@ -259,6 +306,37 @@ LbmStatus lbm_net_input(const void* mask, float inlet, const float* xs, const fl
     inputKernel<<<(unsigned) (depth*height), kThreads, 0, (cudaStream_t) stream>>>((const unsigned char*) mask, inlet, xs, ys,
                                                                                   zs, (uint4*) out, height, width);
     return launched("lbm_net_input");
+}
+
+LbmStatus lbm_net_weights(int layers, const float* const* w, void* const* w16, void* const* wt, const int* cout,
+                          const int* cin, void* stream) {
+    if (layers <= 0 || !w || !w16 || !wt || !cout || !cin)
+        return invalid("lbm_net_weights: null pointer or no layers");
+    for (int i = 0; i < layers; i++)
+        if (!w[i] || !w16[i] || cout[i] <= 0 || cin[i] <= 0)
+            return invalid("lbm_net_weights: null pointer or empty layer");
+    for (int done = 0; done < layers; done += kLayers) {
+        WeightTable t{};
+        const int count = std::min(kLayers, layers - done);
+        long long blocks = 0;
+        for (int i = 0; i < count; i++) {
+            t.w[i] = w[done + i];
+            t.w16[i] = (__nv_bfloat16*) w16[done + i];
+            t.wt[i] = (__nv_bfloat16*) wt[done + i];
+            t.cout[i] = cout[done + i];
+            t.cin[i] = cin[done + i];
+            t.first[i] = (unsigned) blocks;
+            blocks += 27LL*((t.cout[i] + kTile - 1LL)/kTile)*((t.cin[i] + kTile - 1LL)/kTile);
+            if (blocks > 0x7FFFFFFFLL)
+                return invalid("lbm_net_weights: too many weights");
+        }
+        t.first[count] = (unsigned) blocks;
+        weightsKernel<<<(unsigned) blocks, kThreads, 0, (cudaStream_t) stream>>>(t);
+        const LbmStatus status = launched("lbm_net_weights");
+        if (status != LBM_OK)
+            return status;
+    }
+    return LBM_OK;
 }
 
 } // extern "C"

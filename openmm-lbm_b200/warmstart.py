@@ -42,6 +42,7 @@ _SIGNATURES = {
     'lbm_net_upsample_concat': (ctypes.c_int, [ctypes.c_void_p]*3 + [ctypes.c_int]*6 + [ctypes.c_void_p]),
     'lbm_net_upsample_concat_grad': (ctypes.c_int, [ctypes.c_void_p]*3 + [ctypes.c_int]*6 + [ctypes.c_void_p]),
     'lbm_net_relu_bias_grad': (ctypes.c_int, [ctypes.c_void_p]*4 + [ctypes.c_longlong, ctypes.c_int, ctypes.c_void_p]),
+    'lbm_net_weights': (ctypes.c_int, [ctypes.c_int] + [ctypes.c_void_p]*6),
     'lbm_net_input': (ctypes.c_int, [ctypes.c_void_p, ctypes.c_float] + [ctypes.c_void_p]*4 + [ctypes.c_int]*3 +
                       [ctypes.c_void_p]),
 }
@@ -72,11 +73,14 @@ def _volume(t):
 
 def conv3d_forward(x, w, bias=None, relu=False):
     """y = conv3d(x, w) + bias (then ReLU): x (N, cin, D, H, W) BF16 channels-last, w (cout, 27, cin) BF16."""
+    return _forward(x, w.contiguous(), w.shape[0], bias, relu)
+
+
+def _forward(x, w, cout, bias, relu):
+    """conv3d_forward of weights that are contiguous, in whatever shape."""
     lib = _lib()
     x = _volume(x)
     n, cin, d, h, wd = x.shape
-    cout = w.shape[0]
-    w = w.contiguous()
     y = torch.empty((n, cout, d, h, wd), device=x.device, dtype=torch.bfloat16, memory_format=torch.channels_last_3d)
     b = bias.contiguous().float() if bias is not None else None
     check(lib.lbm_conv3d_forward(x.data_ptr(), w.data_ptr(), b.data_ptr() if b is not None else None, y.data_ptr(),
@@ -108,25 +112,55 @@ def conv_status():
     check(lib.lbm_conv3d_status(_stream()), lib)
 
 
+def pack_weights(weights, transposed):
+    """The BF16 weights that the convolutions read, for FP32 weights (cout, 27, cin): per layer a pair of flat tensors, in
+    the layout of conv3d_forward and, where `transposed` says so, flipped and transposed for the input gradient (None
+    elsewhere); one launch for all layers.  None for weights of another kind, which are converted one by one."""
+    device = weights[0].device
+    for w in weights:
+        if not (w.is_cuda and w.dtype == torch.float32 and w.dim() == 3 and w.shape[1] == 27 and w.numel() > 0
+                and w.is_contiguous() and w.device == device):
+            return None
+    lib = _lib()
+    count = len(weights)
+    sizes = [w.numel() for w in weights]
+    parts = sizes + [size for size, t in zip(sizes, transposed) if t]
+    pieces = torch.empty(sum(parts), device=device, dtype=torch.bfloat16).split(parts)
+    flipped = iter(pieces[count:])
+    pairs = [(pieces[i], next(flipped) if transposed[i] else None) for i in range(count)]
+    pointers = ctypes.c_void_p*count
+    ints = ctypes.c_int*count
+    check(lib.lbm_net_weights(count, pointers(*[w.data_ptr() for w in weights]), pointers(*[p.data_ptr() for p, _ in pairs]),
+                              pointers(*[t.data_ptr() if t is not None else None for _, t in pairs]),
+                              ints(*[w.shape[0] for w in weights]), ints(*[w.shape[2] for w in weights]), _stream()), lib)
+    return pairs
+
+
 class Conv3dFunction(torch.autograd.Function):
     """BF16 3x3x3 convolution with FP32 master weights; the ReLU (when set) is fused into the forward kernel and its
     mask taken from the output in the backward pass."""
 
     @staticmethod
-    def forward(ctx, x, weight, bias, relu):
-        w16 = weight.to(torch.bfloat16)
-        y = conv3d_forward(x, w16, bias, relu)
-        ctx.save_for_backward(x, w16, y if relu else None)
-        ctx.relu = relu
+    def forward(ctx, x, weight, bias, relu, packed=None):
+        if packed is None:
+            pairs = pack_weights([weight], [ctx.needs_input_grad[0]])
+            packed = pairs[0] if pairs else (weight.to(torch.bfloat16).contiguous(), None)
+        w16, wt = packed
+        y = _forward(x, w16, weight.shape[0], bias, relu)
+        ctx.save_for_backward(x, w16, wt, y if relu else None)
+        ctx.shape = weight.shape
         return y
 
     @staticmethod
     def backward(ctx, dy):
-        x, w16, y = ctx.saved_tensors
+        x, w16, wt, y = ctx.saved_tensors
         dy, db = relu_bias_grad(dy, y)
-        dx = conv3d_input_grad(dy, w16) if ctx.needs_input_grad[0] else None
+        dx = None
+        if ctx.needs_input_grad[0]:
+            dx = (_forward(dy, wt.contiguous(), ctx.shape[2], None, False) if wt is not None
+                  else conv3d_input_grad(dy, w16.view(ctx.shape)))
         dw = conv3d_weight_grad(x, dy)
-        return dx, dw, db, None
+        return dx, dw, db, None, None
 
 
 def _empty_volume(like, channels, d, h, w):
@@ -236,23 +270,27 @@ class WarmStartNet(torch.nn.Module):
     def parameter_count(self):
         return sum(p.numel() for p in self.weights) + sum(p.numel() for p in self.biases)
 
-    def _conv(self, i, h, relu=True):
-        return Conv3dFunction.apply(h, self.weights[i], self.biases[i], relu)
-
     def forward(self, x):
         levels = len(self.widths)
+        weights, biases = list(self.weights), list(self.biases)
+        grad = torch.is_grad_enabled()
+        packed = pack_weights(weights, [grad and (k > 0 or x.requires_grad) for k in range(len(weights))])
+
+        def conv(k, h, relu=True):
+            return Conv3dFunction.apply(h, weights[k], biases[k], relu, packed[k] if packed else None)
+
         skips, h, i = [], x, 0
         for level in range(levels):
-            h = self._conv(i + 1, self._conv(i, h))
+            h = conv(i + 1, conv(i, h))
             i += 2
             if level < levels - 1:
                 skips.append(h)
                 h = Pool2.apply(h)
         for level in range(levels - 2, -1, -1):
             h = UpsampleConcat.apply(h, skips[level])
-            h = self._conv(i + 1, self._conv(i, h))
+            h = conv(i + 1, conv(i, h))
             i += 2
-        return self._conv(i, h, relu=False)[:, :self.out_channels]
+        return conv(i, h, relu=False)[:, :self.out_channels]
 
 
 # ------------------------------------------------------------------------------------------------------------------

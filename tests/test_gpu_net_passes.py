@@ -70,3 +70,19 @@ def test_network_input_is_that_of_torch():
         got = ws.network_input(masks, 0.013)
         ref = ws.network_input([m.float() for m in masks], 0.013)
         assert torch.equal(got, ref) and got.is_contiguous(memory_format=torch.channels_last_3d)
+
+
+@pytest.mark.parametrize('sizes', [[(16, 8)], [(48, 40), (16, 16), (160, 224), (20, 3)], [(16, 33)]*33])
+def test_packed_weights(sizes):
+    g = torch.Generator(device='cuda')
+    g.manual_seed(8)
+    weights = [torch.randn((cout, 27, cin), device='cuda', generator=g) for cout, cin in sizes]
+    transposed = [i % 2 == 0 for i in range(len(sizes))]
+    for w, t, (w16, wt) in zip(weights, transposed, ws.pack_weights(weights, transposed)):
+        ref = w.to(torch.bfloat16)
+        assert torch.equal(w16, ref.flatten())
+        assert (wt is not None) == t
+        if t:
+            assert torch.equal(wt, ref.flip(1).permute(2, 1, 0).flatten())
+    assert ws.pack_weights([weights[0].transpose(0, 2)], [False]) is None or sizes[0][0] == sizes[0][1]
+    assert ws.pack_weights([weights[0].double()], [False]) is None
