@@ -100,6 +100,7 @@ public:
     long long launches;
 private:
     void launchStreamCollide(long long stepIndex, bool remove, bool react);
+    bool follows(bool react) const;
     void release();            // gives back the device memory and events
     LbmLatticeParameters lattice;
     int storageType;
