@@ -42,6 +42,7 @@ struct FluidView {
     uint32_t seed;
     double mu;                 // 3 kT of the fluid fluctuations in lattice units (0: no fluctuations)
     int faceOpen;              // some face is not periodic
+    int removes;               // some steps remove the fluid's momentum
     const uint32_t* solidMask; // bit per node, rows padded to 32 bits; NULL without solid nodes
     const uint32_t* reactMask; // bit per node with a coupling reaction; NULL without particles
     const void* reaction;      // 4 values (R) per node, lattice units

@@ -22,6 +22,7 @@ def run(shape, precision, solids, open_faces, stream):
     wall = np.repeat(((y == 0) | (y == ny - 1) | (z == 0) | (z == nz - 1)).ravel(), nx)
     kernel = B200Kernel(lattice, [], np.nonzero(wall)[0] if solids else [], precision, stream=stream)
     for step in range(60):
+        kernel.begin_step(step)
         kernel.execute(step)
     return [np.array(kernel.get_fluid_state()), kernel.get_fluid_mach_number()] + [np.array(f) for f in kernel.get_fluid_fields()]
 
