@@ -659,7 +659,9 @@ convSliceKernel(const SliceParams p) {
         }
     }
     else {
-        // ---- epilogue: warp w owns the lanes 32 w .. 32 w + 31 of the accumulators, rows of the tile ----
+        // ---- epilogue: warp w owns the lanes 32 w .. 32 w + 31 of the accumulators, rows of the tile.  A load from tensor
+        // memory needs the whole warp: all lanes take one answer of the wait, and come together again after the stores of
+        // those whose voxel lies in the volume ----
         const int row = warp*32 + lane, vx = row%kTileX, vy = row/kTileX;
         int plane0 = 0;
         bool ok = true;
@@ -669,7 +671,7 @@ convSliceKernel(const SliceParams p) {
             const bool store = xx < p.W && yy < p.H;
             for (int k = 0; k < it.zc; k++) {
                 const int plane = plane0 + k, acc = plane%p.accSlots;
-                ok = waitOrStop(smemAddr(&bars->accFull[acc]), (uint32_t) ((plane/p.accSlots) & 1), limit, stop);
+                ok = warpWait(smemAddr(&bars->accFull[acc]), (uint32_t) ((plane/p.accSlots) & 1), limit, stop);
                 if (!ok)
                     break;
                 fenceAfterSync();
@@ -688,6 +690,7 @@ convSliceKernel(const SliceParams p) {
                         reinterpret_cast<uint4*>(out + col)[0] = reinterpret_cast<const uint4*>(o)[0];
                         reinterpret_cast<uint4*>(out + col)[1] = reinterpret_cast<const uint4*>(o)[1];
                     }
+                    __syncwarp();
                 }
                 fenceBeforeSync();
                 arrive(smemAddr(&bars->accEmpty[acc]));
@@ -697,10 +700,10 @@ convSliceKernel(const SliceParams p) {
     }
     fenceBeforeSync();
     __syncthreads();
-    if (tid == 0 && bars->stop)
-        atomicExch(&convStatus, (int) LBM_ERR_DEVICE_TIMEOUT);
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(ncols) : "memory");
+    if (tid == 0 && bars->stop)
+        atomicExch(&convStatus, (int) LBM_ERR_DEVICE_TIMEOUT);
 }
 
 __global__ void __launch_bounds__(kThreads)
@@ -766,6 +769,7 @@ convForwardKernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __re
                 }
                 *reinterpret_cast<uint4*>(y + mo*cout + col) = *reinterpret_cast<const uint4*>(out);
             }
+            __syncwarp();
         }
     }
     else if (tid == 0)
@@ -1116,10 +1120,10 @@ convSliceGradKernel(const GradParams p) {
     }
     fenceBeforeSync();
     __syncthreads();
-    if (tid == 0 && bars->stop)
-        atomicExch(&convStatus, (int) LBM_ERR_DEVICE_TIMEOUT);
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(ncols) : "memory");
+    if (tid == 0 && bars->stop)
+        atomicExch(&convStatus, (int) LBM_ERR_DEVICE_TIMEOUT);
 }
 
 size_t stageBytes(int rowsB) {
