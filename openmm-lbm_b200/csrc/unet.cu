@@ -792,8 +792,8 @@ convForwardKernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __re
 // buffers, warp 8 issues the MMAs, and warps 9-16 add finished sums to dw with FP32 atomics.
 //
 // The tensor core truncates its running sums: their relative error grows by about 2^-25 per MMA.  So a sum is handed to the
-// atomics (rounded to nearest) after `chain` MMAs at most, and the accumulators are a ring of units (all dz of an MMA, or
-// one) that are read and cleared while the next unit fills.
+// atomics (rounded to nearest) after `chain` MMAs at most (8 to 48, planGradient), and the accumulators are a ring of units
+// (all dz of an MMA, or one) that are read and cleared while the next unit fills.
 //
 // Bound: 16 -> 16 channels read 4 KB of x and 4.6 KB of dy (68 wavefronts of shared memory) per MMA and 16 voxels, 19 us
 // on two 64 x 64 x 128 volumes.  Measured there: 79 us, what remains being the copies (dy three times) and the atomics of
@@ -905,6 +905,8 @@ convSliceGradKernel(const GradParams p) {
         n = i/p.zBlocks;
         zc = min(p.zLen, p.D - z0);
     };
+    // A sum of `chain` MMAs ends with item i where this is the CTA's last or a whole item more could be too much.
+    const int room = p.chain - kRowsY*p.zLen;
 
     if (warp < kGradProducers/32) {
         CopyQueue queue;
@@ -1059,7 +1061,7 @@ convSliceGradKernel(const GradParams p) {
             commitElected(smemAddr(&bars->dyEmpty[buffer]));
             buffer ^= 1;
             chain += rows*zc;
-            if (chain + kRowsY > p.chain || i + (int) gridDim.x >= p.items) {
+            if (chain > room || i + (int) gridDim.x >= p.items) {
                 for (int k = 0; k < unitsPerSum; k++)
                     commitElected(smemAddr(&bars->unitFull[(unit + k)%units]));
                 unit += unitsPerSum;
@@ -1088,7 +1090,7 @@ convSliceGradKernel(const GradParams p) {
             int n, z0, zc, y0, x0;
             item(i, n, z0, zc, y0, x0);
             chain += min(kRowsY, p.H - y0)*zc;
-            if (chain + kRowsY <= p.chain && i + (int) gridDim.x < p.items)
+            if (chain <= room && i + (int) gridDim.x < p.items)
                 continue;
             chain = 0;
             for (int k = 0; k < unitsPerSum && ok; k++) {
@@ -1241,11 +1243,14 @@ size_t planGradient(GradParams& p, int sms, dim3& grid) {
     p.dzCount = p.cout <= 48 ? 3 : 1;
     p.coTile = divisor(p.dzCount == 3 ? 48 : 80);
     p.coBlocks = p.cout/p.coTile;
-    // MMAs per sum: an error of about 1e-6 on large volumes; small ones, whose sums are short anyway, keep theirs at 1e-7.
+    // MMAs per sum: an error of about 1e-6 on large volumes; small ones, whose sums are short anyway, keep theirs at 1e-7
+    // (that takes items of a plane instead of four there: 16 -> 16 at 35 x 40 x 21 16.6 us with sums of 8, 11.7 with 32; at
+    // 16 x 8 x 4 9.3 and 11.4).
     const long long runs = ((long long) p.W*p.H*p.D*p.batch + 15)/16, parts = ((p.cout + 127)/128)*(((long long) 27*p.cin + 255)/256);
     p.chain = (int) std::max(8LL, std::min(p.dzCount == 3 ? 32LL : 48LL, runs/(4*sms/parts + 1)));
-    // Planes per item: as many as keep a buffer of dy within 75 KB (a slice of x is read by up to three planes).
-    p.zLen = p.dzCount == 3 ? std::max(1, std::min(4, 76800/gradDyBytes(p.coTile, 1))) : 1;
+    // Planes per item: as many as keep a buffer of dy within 75 KB (a slice of x is read by up to three planes) and an
+    // item's MMAs within a sum.
+    p.zLen = p.dzCount == 3 ? std::max(1, std::min({4, 76800/gradDyBytes(p.coTile, 1), p.chain/kRowsY})) : 1;
     p.colsX = (p.W + kRunX - 1)/kRunX;
     p.colsY = (p.H + kRowsY - 1)/kRowsY;
     p.zBlocks = (p.D + p.zLen - 1)/p.zLen;
