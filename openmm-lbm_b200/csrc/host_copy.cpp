@@ -41,14 +41,10 @@ HostCopy::~HostCopy() {
             if (e != nullptr)
                 cudaEventDestroy(e);
     }
-    if (ready != nullptr)
-        cudaEventDestroy(ready);
     cudaFreeHost(pinned);
 }
 
 void HostCopy::prepare(int threads) {
-    if (ready == nullptr)
-        check(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming), "cudaEventCreate");
     while ((int) workers.size() < threads) {
         workers.emplace_back();
         Worker& w = workers.back();
@@ -77,9 +73,10 @@ void HostCopy::download(const std::vector<Piece>& pieces, cudaStream_t stream) {
         check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
         return;
     }
+    // The caller's own steps first: others shall not wait for them.
+    check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
     std::lock_guard<std::mutex> lock(busy);
     prepare(threads);
-    check(cudaEventRecord(ready, stream), "cudaEventRecord");
     std::vector<Piece> chunks;
     for (const Piece& p : pieces)
         for (size_t at = 0; at < p.bytes; at += kChunk)
@@ -89,8 +86,6 @@ void HostCopy::download(const std::vector<Piece>& pieces, cudaStream_t stream) {
     auto run = [&](int t) {
         cudaError_t e = cudaSetDevice(device);
         const Worker& w = workers[t];
-        if (e == cudaSuccess)
-            e = cudaStreamWaitEvent(w.stream, ready, 0);
         // A chunk lands in one buffer while the one before it is copied out of the other.
         Piece held[2] = {{nullptr, nullptr, 0}, {nullptr, nullptr, 0}};
         for (int b = 0; e == cudaSuccess && failed.load() == (int) cudaSuccess; b ^= 1) {

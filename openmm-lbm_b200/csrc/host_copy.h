@@ -28,8 +28,8 @@ public:
     static std::shared_ptr<HostCopy> forDevice(int device);
     HostCopy(const HostCopy&) = delete;
     HostCopy& operator=(const HostCopy&) = delete;
-    // Copies the pieces once the work on `stream` is done; returns when they are in place.  One caller at a time: others
-    // wait for their turn (they would share the same link).
+    // Copies the pieces once the work on `stream` is done; returns when they are in place.  The copies themselves take
+    // turns (they would share the same link); a caller waits for its own stream before its turn.
     void download(const std::vector<Piece>& pieces, cudaStream_t stream);
 private:
     struct Worker {
@@ -42,7 +42,6 @@ private:
     std::vector<Worker> workers;
     char* pinned = nullptr;        // two chunks per worker
     int pinnedWorkers = 0;
-    cudaEvent_t ready = nullptr;
 };
 
 } // namespace lbm
