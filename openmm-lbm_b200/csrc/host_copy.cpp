@@ -34,31 +34,43 @@ std::shared_ptr<HostCopy> HostCopy::forDevice(int device) {
 }
 
 HostCopy::~HostCopy() {
-    for (Worker& w : workers) {
-        if (w.stream != nullptr)
-            cudaStreamDestroy(w.stream);
-        for (cudaEvent_t e : w.landed)
-            if (e != nullptr)
-                cudaEventDestroy(e);
-    }
-    cudaFreeHost(pinned);
+    for (Worker& w : workers)
+        release(w);
 }
 
-void HostCopy::prepare(int threads) {
+bool HostCopy::create(Worker& w) {
+    bool ok = cudaStreamCreateWithFlags(&w.stream, cudaStreamNonBlocking) == cudaSuccess;
+    for (cudaEvent_t& e : w.landed)
+        ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+    ok = ok && cudaHostAlloc((void**) &w.pinned, 2*kChunk, cudaHostAllocDefault) == cudaSuccess;
+    if (!ok) {
+        cudaGetLastError();        // the copy goes another way: later calls shall not find this error
+        release(w);
+    }
+    return ok;
+}
+
+void HostCopy::release(Worker& w) {
+    if (w.stream != nullptr)
+        cudaStreamDestroy(w.stream);
+    for (cudaEvent_t e : w.landed)
+        if (e != nullptr)
+            cudaEventDestroy(e);
+    if (w.pinned != nullptr)
+        cudaFreeHost(w.pinned);
+    w = Worker();
+}
+
+// The workers there are, `threads` of them if they can be had.
+int HostCopy::prepare(int threads) {
     while ((int) workers.size() < threads) {
-        workers.emplace_back();
-        Worker& w = workers.back();
-        check(cudaStreamCreateWithFlags(&w.stream, cudaStreamNonBlocking), "cudaStreamCreate");
-        for (cudaEvent_t& e : w.landed)
-            check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+        Worker w;
+        workers.reserve(workers.size() + 1);
+        if (!create(w))
+            break;
+        workers.push_back(w);
     }
-    if (pinnedWorkers < threads) {
-        cudaFreeHost(pinned);
-        pinned = nullptr;
-        pinnedWorkers = 0;
-        check(cudaHostAlloc((void**) &pinned, 2*kChunk*threads, cudaHostAllocDefault), "cudaHostAlloc");
-        pinnedWorkers = threads;
-    }
+    return std::min(threads, (int) workers.size());
 }
 
 void HostCopy::download(const std::vector<Piece>& pieces, cudaStream_t stream) {
@@ -66,17 +78,22 @@ void HostCopy::download(const std::vector<Piece>& pieces, cudaStream_t stream) {
     for (const Piece& p : pieces)
         total += p.bytes;
     const int cores = std::max(1, (int) std::thread::hardware_concurrency());
-    const int threads = std::min({kMaxThreads, cores, (int) std::min<size_t>(kMaxThreads, total/kBytesPerThread)});
+    int threads = std::min({kMaxThreads, cores, (int) std::min<size_t>(kMaxThreads, total/kBytesPerThread)});
+    std::unique_lock<std::mutex> lock(busy, std::defer_lock);
+    if (threads >= 2) {
+        // The caller's own steps first: others shall not wait for them.
+        check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
+        lock.lock();
+        threads = prepare(threads);
+    }
     if (threads < 2) {
+        if (lock.owns_lock())
+            lock.unlock();
         for (const Piece& p : pieces)
             check(cudaMemcpyAsync(p.host, p.device, p.bytes, cudaMemcpyDeviceToHost, stream), "cudaMemcpyAsync");
         check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
         return;
     }
-    // The caller's own steps first: others shall not wait for them.
-    check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
-    std::lock_guard<std::mutex> lock(busy);
-    prepare(threads);
     std::vector<Piece> chunks;
     for (const Piece& p : pieces)
         for (size_t at = 0; at < p.bytes; at += kChunk)
@@ -90,7 +107,7 @@ void HostCopy::download(const std::vector<Piece>& pieces, cudaStream_t stream) {
         Piece held[2] = {{nullptr, nullptr, 0}, {nullptr, nullptr, 0}};
         for (int b = 0; e == cudaSuccess && failed.load() == (int) cudaSuccess; b ^= 1) {
             const size_t i = next.fetch_add(1);
-            char* buffer = pinned + (2*(size_t) t + b)*kChunk;
+            char* buffer = w.pinned + b*kChunk;
             held[b].host = nullptr;
             if (i < chunks.size()) {
                 held[b] = chunks[i];
@@ -102,7 +119,7 @@ void HostCopy::download(const std::vector<Piece>& pieces, cudaStream_t stream) {
             if (e == cudaSuccess && before.host != nullptr) {
                 e = cudaEventSynchronize(w.landed[b ^ 1]);
                 if (e == cudaSuccess)
-                    std::memcpy(before.host, pinned + (2*(size_t) t + (b ^ 1))*kChunk, before.bytes);
+                    std::memcpy(before.host, w.pinned + (b ^ 1)*kChunk, before.bytes);
                 before.host = nullptr;
             }
             if (held[b].host == nullptr)

@@ -29,19 +29,21 @@ public:
     HostCopy(const HostCopy&) = delete;
     HostCopy& operator=(const HostCopy&) = delete;
     // Copies the pieces once the work on `stream` is done; returns when they are in place.  The copies themselves take
-    // turns (they would share the same link); a caller waits for its own stream before its turn.
+    // turns (they would share the same link); a caller waits for its own stream before its turn.  Without pinned memory,
+    // streams or events for two threads the copy is a plain one.
     void download(const std::vector<Piece>& pieces, cudaStream_t stream);
 private:
     struct Worker {
         cudaStream_t stream = nullptr;
         cudaEvent_t landed[2] = {nullptr, nullptr};
+        char* pinned = nullptr;    // two chunks
     };
-    void prepare(int threads);
+    static bool create(Worker& worker);
+    static void release(Worker& worker);
+    int prepare(int threads);
     const int device;
     std::mutex busy;
     std::vector<Worker> workers;
-    char* pinned = nullptr;        // two chunks per worker
-    int pinnedWorkers = 0;
 };
 
 } // namespace lbm

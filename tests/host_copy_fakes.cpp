@@ -1,6 +1,6 @@
 // csrc/host_copy.cpp against stand-ins for the CUDA calls that it makes, so that its threads, its lock and its failures can
 // be tested without a GPU (tests/test_host_copy.py builds and runs this).  A stream is a flag that holds its waiters back;
-// copies are made at once, and a chosen one fails.  Exits with 0, or prints what went wrong.
+// copies are made at once; the calls of one kind fail from a chosen one on.  Exits with 0, or prints what went wrong.
 #include "host_copy.h"
 #include <atomic>
 #include <chrono>
@@ -17,7 +17,8 @@ struct CUevent_st {
     CUstream_st* stream = nullptr;
 };
 
-static std::atomic<int> copies(0), failCopy(-1), live(0);
+static std::atomic<int> hostAllocs(0), failFrom(1 << 30), streams(0), failStream(-1), copies(0), failCopy(-1);
+static std::atomic<int> live(0);
 
 static cudaError_t wait(CUstream_st* s) {
     for (int i = 0; i < 20000 && s != nullptr; i++) {
@@ -34,6 +35,8 @@ cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t) { return "made up"; }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
+    if (streams++ == failStream)
+        return cudaErrorMemoryAllocation;
     live++;
     *s = new CUstream_st;
     return cudaSuccess;
@@ -42,6 +45,9 @@ cudaError_t cudaStreamDestroy(cudaStream_t s) { live--; delete s; return cudaSuc
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { live++; *e = new CUevent_st; return cudaSuccess; }
 cudaError_t cudaEventDestroy(cudaEvent_t e) { live--; delete e; return cudaSuccess; }
 cudaError_t cudaHostAlloc(void** p, size_t bytes, unsigned) {
+    const int i = hostAllocs++;
+    if (i >= failFrom)
+        return cudaErrorMemoryAllocation;
     live++;
     *p = std::malloc(bytes);
     return cudaSuccess;
@@ -118,6 +124,24 @@ int main() {
         slow.held = false;
         other.join();
         mine.join();
+    }
+    // Without pinned memory, with some of it, and once there is some again.
+    for (int some : {0, 1, 3}) {
+        lbm::HostCopy copier(0);
+        failFrom = hostAllocs + some;
+        copyTwo(copier, stream, 40*kMB, "a copy without pinned memory went wrong");
+        failFrom = 1 << 30;
+        copyTwo(copier, stream, 40*kMB, "a copy after the pinned memory ran out went wrong");
+    }
+    {
+        lbm::HostCopy copier(0);
+        failStream = streams + 1;
+        try {
+            copyTwo(copier, stream, 40*kMB, "a copy with too few streams went wrong");
+        }
+        catch (const lbm::Error&) {
+        }
+        copyTwo(copier, stream, 40*kMB, "a copy after a stream failed went wrong");
     }
     {
         // A copy that fails is reported, and the next one works.

@@ -1,6 +1,6 @@
 """The copies of fields and state to the host (csrc/host_copy.cpp) against stand-ins for the CUDA calls, without a GPU: the
-bytes of every size and number of threads; a kernel whose steps are still queued does not hold up the read-out of another; a
-copy that fails."""
+bytes of every size and number of threads; a kernel whose steps are still queued does not hold up the read-out of another;
+pinned memory, streams or copies that fail."""
 import os
 import subprocess
 
