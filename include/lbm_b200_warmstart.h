@@ -42,8 +42,10 @@ LbmStatus lbm_conv3d_set_wait_limit(long long polls);
  *   pool             y = mean of the 2 x 2 x 2 windows of x (a last odd plane is left out), and its gradient (dx of a left
  *                    out plane is not written)
  *   upsample_concat  y = the nearest 2x upsampling of x, then skip, along the channels (even sizes), and its gradients
- *   relu_bias_grad   out = dy where y > 0 and 0 dy elsewhere, db[channels] += its sums over the voxels (FP32); with y NULL
- *                    the sums of dy alone
+ *   relu_bias_grad   out = dy where y > 0 and 0 dy elsewhere, db[channels] += its sums over the voxels (FP32, in an order
+ *                    of their own: the same bits every time); with y NULL the sums of dy alone.  The _with form stores
+ *                    db instead of adding to it and takes the lbm_net_relu_bias_scratch() bytes of device memory that the
+ *                    sums need (aligned to 4 bytes); the other takes them from the device's default memory pool
  *   weights          of every layer the FP32 weights w[cout][27][cin] in BF16, and where wt[layer] is not NULL flipped and
  *                    transposed, wt[cin][26 - tap][cout]; the tables are host memory, no alignment is asked for
  *   input            the network's input for one solid mask (bytes): mask, inlet, xs[x], ys[y], zs[z] and three zeros per
@@ -57,6 +59,9 @@ LbmStatus lbm_net_upsample_concat_grad(const void* dy, void* dx, void* dskip, in
                                        int channels, int skip_channels, void* stream);
 LbmStatus lbm_net_relu_bias_grad(const void* dy, const void* y, void* out, float* db, long long voxels, int channels,
                                  void* stream);
+size_t lbm_net_relu_bias_scratch(long long voxels, int channels);   /* 0: sizes that the calls refuse */
+LbmStatus lbm_net_relu_bias_grad_with(const void* dy, const void* y, void* out, float* db, float* scratch, long long voxels,
+                                      int channels, void* stream);
 LbmStatus lbm_net_weights(int layers, const float* const* w, void* const* w16, void* const* wt, const int* cout,
                           const int* cin, void* stream);
 LbmStatus lbm_net_input(const void* mask, float inlet, const float* xs, const float* ys, const float* zs, void* out,

@@ -4,7 +4,7 @@
 // each reads and writes every volume once, in the layout the convolutions use.  The library passes that they stand in for
 // worked in planar order between layout copies.  Per training step on two 64 x 64 x 128 volumes: upsampling with the
 // concatenation 43 us (262, and the copies around it), its gradients 37 us (140 and copies), the ReLU's and biases'
-// gradients of 15 layers 138 us (980 in five passes), pooling 9 us (56), the input 5 us per mask (twelve launches).
+// gradients of 15 layers 132 us (980 in five passes), pooling 9 us (56), the input 5 us per mask (twelve launches).
 #include "lbm_b200_warmstart.h"
 #include "lbm_internal.h"
 #include <cuda_bf16.h>
@@ -134,41 +134,90 @@ upsampleConcatGradKernel(const uint4* __restrict__ dy, uint4* __restrict__ dx, u
 }
 
 // The gradient of a layer's output before its ReLU, dy (y > 0) (y == nullptr: no ReLU, and out is not written), and its
-// sums over the voxels added to db: a thread keeps one channel group and adds up its voxels, a block its threads.
+// sums over the voxels: a thread keeps one channel group and adds up its voxels, a block its threads as a tree, and
+// biasSumKernel the blocks, in their order, so that the sums are the same bits every time.  Bound by the volumes' bytes, read
+// and written once.  592 blocks, two voxels of a thread in flight: 16 channels on two 64 x 64 x 128 volumes 15.0 us (18.6 with
+// one voxel and FP32 atomics into zeroed sums; four in flight 5 us more than two, 1184 blocks 5 us more than 592), 160
+// channels at 8 x 8 x 16 4.9 us (3.7).  A ticket, by which the last block adds the blocks' sums, costs more than the second
+// launch does: 24.6 and 12.5 us.
+constexpr int kBiasBlocks = 592, kBiasAhead = 2;
+
+// Leaves in the rows of part 0 the sums of `parts` rows of `stride` elements, added as a tree (thread part*stride + i holds
+// element i of a row, kThreads apart for each of the N sums).
+template <int N>
+__device__ __forceinline__ void treeSum(float* sums, int part, int parts, int stride) {
+    for (int h = parts > 1 ? 1 << (31 - __clz(parts - 1)) : 0; h > 0; h /= 2) {
+        __syncthreads();
+        if (part < h && part + h < parts)
+#pragma unroll
+            for (int k = 0; k < N; k++)
+                sums[k*kThreads + threadIdx.x] += sums[k*kThreads + threadIdx.x + h*stride];
+    }
+    __syncthreads();
+}
+
 __global__ void __launch_bounds__(kThreads)
-reluBiasGradKernel(const uint4* __restrict__ dy, const uint4* __restrict__ y, uint4* __restrict__ out, float* __restrict__ db,
-                   size_t voxels, int groups) {
-    extern __shared__ float sums[];                       // [threads][8]
+reluBiasGradKernel(const uint4* __restrict__ dy, const uint4* __restrict__ y, uint4* __restrict__ out,
+                   float* __restrict__ partials, size_t voxels, int groups) {
+    __shared__ float sums[8*kThreads];
     const int lanes = kThreads/groups;                    // voxels a block takes at a time
-    const int g = threadIdx.x%groups, lane = threadIdx.x/groups;
+    const int g = threadIdx.x%groups, lane = threadIdx.x/groups, channels = 8*groups;
     float s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    const size_t step = (size_t) gridDim.x*lanes;
     if (lane < lanes)
-        for (size_t v = (size_t) blockIdx.x*lanes + lane; v < voxels; v += (size_t) gridDim.x*lanes) {
-            const uint4 word = __ldg(dy + v*groups + g);
-            float f[8];
-            unpack(word, f);
-            if (y != nullptr) {
-                float a[8];
-                unpack(__ldg(y + v*groups + g), a);
+        for (size_t v = (size_t) blockIdx.x*lanes + lane; v < voxels; v += kBiasAhead*step) {
+            // The loads of several voxels in flight, then their sums in the voxels' order.
+            uint4 word[kBiasAhead], act[kBiasAhead];
 #pragma unroll
-                for (int k = 0; k < 8; k++)
-                    f[k] = a[k] > 0.0f ? f[k] : 0.0f*f[k];
-                out[v*groups + g] = pack(f);
-            }
+            for (int a = 0; a < kBiasAhead; a++)
+                if (v + a*step < voxels) {
+                    word[a] = __ldg(dy + (v + a*step)*groups + g);
+                    if (y != nullptr)
+                        act[a] = __ldg(y + (v + a*step)*groups + g);
+                }
 #pragma unroll
-            for (int k = 0; k < 8; k++)
-                s[k] += f[k];
+            for (int a = 0; a < kBiasAhead; a++)
+                if (v + a*step < voxels) {
+                    float f[8];
+                    unpack(word[a], f);
+                    if (y != nullptr) {
+                        float on[8];
+                        unpack(act[a], on);
+#pragma unroll
+                        for (int k = 0; k < 8; k++)
+                            f[k] = on[k] > 0.0f ? f[k] : 0.0f*f[k];
+                        out[(v + a*step)*groups + g] = pack(f);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 8; k++)
+                        s[k] += f[k];
+                }
         }
 #pragma unroll
     for (int k = 0; k < 8; k++)
-        sums[threadIdx.x*8 + k] = s[k];
-    __syncthreads();
-    for (int c = threadIdx.x; c < 8*groups; c += blockDim.x) {
-        float total = 0;
-        for (int l = 0; l < lanes; l++)
-            total += sums[(l*groups + c/8)*8 + c%8];
-        atomicAdd(db + c, total);
-    }
+        sums[k*kThreads + threadIdx.x] = s[k];
+    treeSum<8>(sums, lane, lanes, groups);
+    for (int c = threadIdx.x; c < channels; c += kThreads)
+        partials[(size_t) blockIdx.x*channels + c] = sums[(c%8)*kThreads + c/8];
+}
+
+// db = (or with `add` +=) the blocks' sums, of 8 channels per block, in their order.
+__global__ void __launch_bounds__(kThreads)
+biasSumKernel(const float* __restrict__ partials, int blocks, int channels, float* __restrict__ db, bool add) {
+    __shared__ float sums[kThreads];
+    const int c = blockIdx.x*8 + threadIdx.x%8, part = threadIdx.x/8;
+    constexpr int parts = kThreads/8;
+    float t[4] = {0, 0, 0, 0};
+#pragma unroll 5
+    for (int b = part; b < blocks; b += 4*parts)
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (b + j*parts < blocks)
+                t[j] += __ldg(partials + (size_t) (b + j*parts)*channels + c);
+    sums[threadIdx.x] = (t[0] + t[1]) + (t[2] + t[3]);
+    treeSum<1>(sums, part, parts, 8);
+    if (part == 0)
+        db[c] = add ? db[c] + sums[threadIdx.x] : sums[threadIdx.x];
 }
 
 // The network's input for one mask: solid, scaled inlet and the coordinates along x, y, z, then zeros; 8 channels a voxel.
@@ -248,6 +297,21 @@ bool rowsFit(int batch, int depth, int height) {
     return batch > 0 && depth > 0 && height > 0 && (long long) batch*depth*height < (1LL << 31);
 }
 
+// Blocks of the bias gradient: two voxels per thread at least.
+int biasBlocks(long long voxels, int channels) {
+    const long long lanes = 2*(kThreads/(channels/8));
+    return (int) std::min<long long>(kBiasBlocks, (voxels + lanes - 1)/lanes);
+}
+
+LbmStatus reluBiasGrad(const void* dy, const void* y, void* out, float* db, bool add, float* scratch, long long voxels,
+                       int channels, cudaStream_t stream) {
+    const int blocks = biasBlocks(voxels, channels);
+    reluBiasGradKernel<<<(unsigned) blocks, kThreads, 0, stream>>>((const uint4*) dy, (const uint4*) y, (uint4*) out, scratch,
+                                                                   (size_t) voxels, channels/8);
+    biasSumKernel<<<(unsigned) (channels/8), kThreads, 0, stream>>>(scratch, blocks, channels, db, add);
+    return launched("lbm_net_relu_bias_grad");
+}
+
 } // namespace
 
 extern "C" {
@@ -288,15 +352,33 @@ LbmStatus lbm_net_upsample_concat_grad(const void* dy, void* dx, void* dskip, in
     return launched("lbm_net_upsample_concat_grad");
 }
 
+size_t lbm_net_relu_bias_scratch(long long voxels, int channels) {
+    if (voxels <= 0 || channels <= 0 || channels%8 != 0 || channels > 8*kThreads)
+        return 0;
+    return sizeof(float)*(size_t) biasBlocks(voxels, channels)*channels;
+}
+
+LbmStatus lbm_net_relu_bias_grad_with(const void* dy, const void* y, void* out, float* db, float* scratch, long long voxels,
+                                      int channels, void* stream) {
+    if (!dy || !db || !scratch || (y && !out) || lbm_net_relu_bias_scratch(voxels, channels) == 0)
+        return invalid("lbm_net_relu_bias_grad_with: null pointer, empty volume or channels not a multiple of 8");
+    return reluBiasGrad(dy, y, out, db, false, scratch, voxels, channels, (cudaStream_t) stream);
+}
+
 LbmStatus lbm_net_relu_bias_grad(const void* dy, const void* y, void* out, float* db, long long voxels, int channels,
                                  void* stream) {
-    if (!dy || !db || (y && !out) || voxels <= 0 || channels <= 0 || channels%8 != 0 || channels > 8*kThreads)
+    const size_t bytes = lbm_net_relu_bias_scratch(voxels, channels);
+    if (!dy || !db || (y && !out) || bytes == 0)
         return invalid("lbm_net_relu_bias_grad: null pointer, empty volume or channels not a multiple of 8");
-    const int groups = channels/8, lanes = kThreads/groups;
-    const long long blocks = std::min<long long>(592, (voxels + lanes - 1)/lanes);
-    reluBiasGradKernel<<<(unsigned) blocks, kThreads, kThreads*8*sizeof(float), (cudaStream_t) stream>>>(
-        (const uint4*) dy, (const uint4*) y, (uint4*) out, db, (size_t) voxels, groups);
-    return launched("lbm_net_relu_bias_grad");
+    float* scratch = nullptr;
+    const cudaError_t e = cudaMallocAsync((void**) &scratch, bytes, (cudaStream_t) stream);
+    if (e != cudaSuccess) {
+        lbm::setLastError(std::string("lbm_net_relu_bias_grad: ") + cudaGetErrorString(e));
+        return LBM_ERR_CUDA;
+    }
+    const LbmStatus status = reluBiasGrad(dy, y, out, db, true, scratch, voxels, channels, (cudaStream_t) stream);
+    cudaFreeAsync(scratch, (cudaStream_t) stream);
+    return status;
 }
 
 LbmStatus lbm_net_input(const void* mask, float inlet, const float* xs, const float* ys, const float* zs, void* out,

@@ -41,7 +41,9 @@ _SIGNATURES = {
     'lbm_net_pool_grad': (ctypes.c_int, [ctypes.c_void_p]*2 + [ctypes.c_int]*5 + [ctypes.c_void_p]),
     'lbm_net_upsample_concat': (ctypes.c_int, [ctypes.c_void_p]*3 + [ctypes.c_int]*6 + [ctypes.c_void_p]),
     'lbm_net_upsample_concat_grad': (ctypes.c_int, [ctypes.c_void_p]*3 + [ctypes.c_int]*6 + [ctypes.c_void_p]),
+    'lbm_net_relu_bias_scratch': (ctypes.c_size_t, [ctypes.c_longlong, ctypes.c_int]),
     'lbm_net_relu_bias_grad': (ctypes.c_int, [ctypes.c_void_p]*4 + [ctypes.c_longlong, ctypes.c_int, ctypes.c_void_p]),
+    'lbm_net_relu_bias_grad_with': (ctypes.c_int, [ctypes.c_void_p]*5 + [ctypes.c_longlong, ctypes.c_int, ctypes.c_void_p]),
     'lbm_net_weights': (ctypes.c_int, [ctypes.c_int] + [ctypes.c_void_p]*6),
     'lbm_net_input': (ctypes.c_int, [ctypes.c_void_p, ctypes.c_float] + [ctypes.c_void_p]*4 + [ctypes.c_int]*3 +
                       [ctypes.c_void_p]),
@@ -174,13 +176,15 @@ def relu_bias_grad(dy, y=None):
     lib = _lib()
     dy = _volume(dy.to(torch.bfloat16))
     channels = dy.shape[1]
-    db = torch.zeros(channels, device=dy.device, dtype=torch.float32)
+    voxels = dy.numel()//channels
+    db = torch.empty(channels, device=dy.device, dtype=torch.float32)
+    scratch = torch.empty(lib.lbm_net_relu_bias_scratch(voxels, channels), device=dy.device, dtype=torch.uint8)
     out = dy
     if y is not None:
         y = _volume(y)
         out = torch.empty_like(dy)
-    check(lib.lbm_net_relu_bias_grad(dy.data_ptr(), y.data_ptr() if y is not None else None, out.data_ptr(), db.data_ptr(),
-                                     dy.numel()//channels, channels, _stream()), lib)
+    check(lib.lbm_net_relu_bias_grad_with(dy.data_ptr(), y.data_ptr() if y is not None else None, out.data_ptr(),
+                                          db.data_ptr(), scratch.data_ptr(), voxels, channels, _stream()), lib)
     return out, db
 
 
