@@ -70,7 +70,12 @@ def _stream():
 
 def _volume(t):
     """(N, C, D, H, W) tensor with channels-last storage, as the kernels address it ([n][d][h][w][c])."""
-    return t.contiguous(memory_format=torch.channels_last_3d)
+    return _aligned(t.contiguous(memory_format=torch.channels_last_3d))
+
+
+def _aligned(t):
+    """The tensor at an address that the kernels' 16-byte loads take: a view into a buffer may start anywhere."""
+    return t if t.data_ptr() % 16 == 0 else t.clone()
 
 
 def conv3d_forward(x, w, bias=None, relu=False):
@@ -81,7 +86,7 @@ def conv3d_forward(x, w, bias=None, relu=False):
 def _forward(x, w, cout, bias, relu):
     """conv3d_forward of weights that are contiguous, in whatever shape."""
     lib = _lib()
-    x = _volume(x)
+    x, w = _volume(x), _aligned(w)
     n, cin, d, h, wd = x.shape
     y = torch.empty((n, cout, d, h, wd), device=x.device, dtype=torch.bfloat16, memory_format=torch.channels_last_3d)
     b = bias.contiguous().float() if bias is not None else None
