@@ -18,6 +18,7 @@ which writes it beside itself (weights.pt).
 import argparse
 import ctypes
 import json
+import numbers
 import threading
 import time
 
@@ -344,7 +345,9 @@ def network_input(masks, inlet=0.02):
     n = len(masks)
     nz, ny, nx = masks[0].shape
     dev = masks[0].device
-    if all(m.is_cuda and m.dtype == torch.bool and tuple(m.shape) == (nz, ny, nx) and m.device == dev for m in masks):
+    # The kernel takes non-empty masks on the current device and one number for the inlet; torch anything that broadcasts.
+    if (all(m.is_cuda and m.dtype == torch.bool and tuple(m.shape) == (nz, ny, nx) and m.device == dev for m in masks)
+            and masks[0].numel() > 0 and isinstance(inlet, numbers.Real) and dev.index == torch.cuda.current_device()):
         lib = _lib()
         axes = [torch.linspace(0, 1, k, device=dev) for k in (nx, ny, nz)]
         x = torch.empty((n, IN_CHANNELS, nz, ny, nx), device=dev, dtype=torch.bfloat16,
