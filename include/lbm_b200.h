@@ -97,7 +97,12 @@ typedef struct LbmOptions {
  * positions (nm), velocities (nm/ps) and forces (kJ/mol/nm), 3 doubles per particle, either all in
  * host memory or all in device memory of the handle's device.  lbm_begin_step() may reverse
  * velocities (reflection at walls); lbm_execute() adds the coupling forces to forces, and with the
- * centred drag reads the other forces already accumulated there (LBMForce must be the last force).
+ * centred drag reads the other forces already accumulated there (LBMForce must be the last force).  The positions of a
+ * step are those given to its lbm_begin_step() (to lbm_execute() where that was given none).
+ *
+ * Device arrays are read and written in place by work on the handle's stream (lbm_get_stream()), which a call may leave
+ * queued when it returns: velocities and forces must stay as they are until that work is done, and a caller that changes
+ * or reads the arrays on another stream orders that stream with the handle's.
  */
 typedef struct LbmParticleArrays {
     double* positions;

@@ -373,6 +373,7 @@ batchPairKernel(const ReplicaTable* __restrict__ table, const int* __restrict__ 
         pairForce<false>(table[particleReplica[p]], pp, pos, p, lane, fpair);
 }
 
+// Leapfrog of every bead with the bead forces plus the drag: v += dt F/m, x += dt v (the bead dynamics' integrator).
 __global__ void __launch_bounds__(kBatchThreads)
 batchLeapfrogKernel(const ReplicaTable* __restrict__ table, const int* __restrict__ particleReplica, int totalParticles,
                     const double* __restrict__ invMass, const double* __restrict__ fpair, const double* __restrict__ fdrag,
@@ -483,9 +484,9 @@ __global__ void batchGatherKernel(const T* __restrict__ A, FluidView f, double* 
 // phases of a step separated by bounded grid barriers (grid_barrier.cuh):
 //
 //   phase 1  the sums of the previous step per replica (blocks over replicas: mass, momentum and the velocity that this
-//            step's momentum removal subtracts), bead pair forces and stencil slots (a warp
-//            per bead) with the nodes' j/rho before the removal, and the clear of the previous step's reactions
-//            (their slot nodes are kept in the other half of slotNode)
+//            step's momentum removal subtracts), bead pair forces and stencil slots (a warp per bead) with the nodes'
+//            j/rho before the removal, and the clear of the previous step's reactions (their slot nodes are kept in the
+//            other half of slotNode)
 //   phase 2  explicit drag of every bead (the removal applied to the interpolated velocity: sum w (j/rho - ucm) =
 //            sum w j/rho - ucm sum w) and its reaction on the fluid (warps over beads), then the bead's leapfrog
 //   phase 3  the dense step of every replica (work items of BT nodes), per-warp partial sums

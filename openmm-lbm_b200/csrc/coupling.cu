@@ -41,10 +41,10 @@ const int kThreads = 256;
 
 // The stencil pass: the axis indices and weights of each particle, then one thread per (particle, stencil slot) in
 // two passes: nodes, weights and the moments of each node once, then the moments of every slot.
-// One thread per particle: the node indices and weights of its stencil on each axis, and the first index on each.
+
 // The node indices and weights of every particle's stencil on each axis (entries past the width: index -1, weight 0), 16
 // threads per particle, one per entry: with a thread per particle its twelve kernel values in double came one after
-// another (8.1 -> 3.0 us for 6,400 particles with Keys).
+// another (8.1 -> 3.0 us for 6,400 particles with Keys).  Also the first index on each axis.
 __global__ void stencilAxesKernel(CouplingView c, const double* __restrict__ pos, int4* axisIndex, double2* axisWeight,
                                   int4* firstIndex) {
     const int lane = threadIdx.x & 31, half = lane >> 4, entry = lane & 15;

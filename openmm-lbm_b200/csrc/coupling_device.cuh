@@ -153,15 +153,10 @@ __device__ void pullMomentsAt(const T* A, const FluidView& f, int x, int y, int 
     dr = d; jx = a; jy = b; jz = c;
 }
 
-template <typename T>
-__device__ void pullMoments(const T* A, const FluidView& f, long long node, double& dr, double& jx, double& jy, double& jz) {
-    long long r = node/f.nx;
-    pullMomentsAt<T>(A, f, (int) (node%f.nx), (int) (r%f.ny), (int) (r/f.ny), dr, jx, jy, jz);
-}
-
 // Entry k = lane % 4 of axis lane/4 % 4 (the last group repeats axis 2) of particle i's stencil (LBMStencils::axisWeights,
-// LBMStencils.h:73-95: clamped at open faces, repeated nodes merged into their first entry); lanes 12 and on of a group of 16 hold nothing of use.  Entries past the width: a negative index, weight 0.
-// Called by a whole warp.  COHERENT: the positions were written by the same launch.
+// LBMStencils.h:73-95: clamped at open faces, repeated nodes merged into their first entry); lanes 12 and on of a group of
+// 16 hold nothing of use.  Entries past the width: a negative index, weight 0.  Called by a whole warp.  COHERENT: the
+// positions were written by the same launch.
 template <bool COHERENT>
 __device__ __forceinline__ void stencilEntry(const CouplingView& c, const double* __restrict__ pos, int i, int lane, int& index,
                                              double& weight) {
@@ -202,10 +197,10 @@ __device__ __forceinline__ void stencilEntry(const CouplingView& c, const double
 
 // The stencil slots t = i*slots + s of particle i by one warp: the node and weight of each slot (LBMStencils::axisWeights,
 // LBMStencils.h:73-95) and u = j/rho of the node pulled from the populations (after the momentum removal, :539, :672; a
-// solid node has rho = 0).  Lane 4 a + k < 12 forms entry k of axis a (stencilEntry), and each slot's lane takes its three entries by shuffles: a thread per slot formed all its particle's
-// entries again, nine to twelve kernel values in double with their roots, for the three that it uses (47 us per step of
-// 10,530 beads with the three-point stencil).  COHERENT: the positions were written by the same launch (a persistent
-// kernel): they are read through L2.
+// solid node has rho = 0).  Lane 4 a + k < 12 forms entry k of axis a (stencilEntry), and each slot's lane takes its three
+// entries by shuffles: a thread per slot formed all its particle's entries again, nine to twelve kernel values in double
+// with their roots, for the three that it uses (47 us per step of 10,530 beads with the three-point stencil).  COHERENT:
+// the positions were written by the same launch (a persistent kernel): they are read through L2.
 template <typename T, typename R, bool COHERENT = false>
 __device__ __forceinline__ void stencilParticle(const T* __restrict__ A, const FluidView& f, const CouplingView& c,
                                                 const double* __restrict__ pos, int i, int lane, int remove,
@@ -247,7 +242,7 @@ __device__ __forceinline__ void stencilParticle(const T* __restrict__ A, const F
 }
 
 // The node and weight of stencil slot t, as stencilParticle (from the particle's axis indices and weights, computed once
-// per particle by stencilAxes), with the moments computed once per node: the first slot of a fluid node to claim it in
+// per particle by stencilAxesKernel), with the moments computed once per node: the first slot of a fluid node to claim it in
 // this pass (nodeStamp[node] set to `stamp`) pulls the node's moments into nodeU[node]; stencilGatherSlot then copies
 // them to every slot of the node.  The moments of a node are the same for all its slots, and overlapping stencils
 // share most of their nodes.  With `mark` (the fluid's reaction mask, for the pass of a step) the claiming slot also

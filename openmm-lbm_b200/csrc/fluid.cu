@@ -1404,7 +1404,8 @@ void FluidEngine::clearReactMask(cudaStream_t s) {
 
 // Whether the kernels of a step follow one another as programmatic dependents.  Not in a step with particles, whose
 // kernels follow those of the coupling and whose arrays the host waits for: such a launch costs the host more
-// (32^3 with 64 particles and host arrays: 50 steps 5.0 ms, 4.9 in the plain order).  On the legacy default stream and under capture the plain order is kept.
+// (32^3 with 64 particles and host arrays: 50 steps 5.0 ms, 4.9 in the plain order).  On the legacy default stream and
+// under capture the plain order is kept.
 bool FluidEngine::follows(bool react) const {
     if ((react && reactionDev != nullptr) || stream == nullptr || stream == cudaStreamLegacy)
         return false;

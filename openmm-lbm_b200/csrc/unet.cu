@@ -7,9 +7,9 @@
 //  convSliceGradKernel  dW[cout][k] = sum_voxels dy[voxel][cout] A[voxel][k], the K dimension of the GEMMs being the
 //                       voxels, from slices of x and shifted copies of dy; results added with FP32 atomics
 //
-// The GEMM core of the gathering kernel: 128 x N tiles, K in stages of 64 BF16 (one 128-byte row).  All 128 threads gather a stage into
-// shared memory in the canonical K-major layout with the 128-byte swizzle (8-row atoms of 128-byte rows, the 16-byte
-// chunk index XOR the row within the atom), make it visible to the tensor core's proxy, and one thread issues four
+// The GEMM core of the gathering kernel: 128 x N tiles, K in stages of 64 BF16 (one 128-byte row).  All 128 threads gather
+// a stage into shared memory in the canonical K-major layout with the 128-byte swizzle (8-row atoms of 128-byte rows, the
+// 16-byte chunk index XOR the row within the atom), make it visible to the tensor core's proxy, and one thread issues four
 // tcgen05.mma (K = 16 each, BF16 x BF16 -> FP32 in tensor memory) and commits them to an mbarrier that every
 // thread waits on (bounded: a wait that gives up sets the status flag and the CTA leaves after freeing its tensor
 // memory).  The epilogue reads the accumulators with tcgen05.ld (warp w owns lanes 32w..32w+31 = rows of the tile).
