@@ -17,6 +17,7 @@ which writes it beside itself (weights.pt).
 """
 import argparse
 import ctypes
+import functools
 import json
 import numbers
 import threading
@@ -81,13 +82,13 @@ def _aligned(t):
 
 def conv3d_forward(x, w, bias=None, relu=False):
     """y = conv3d(x, w) + bias (then ReLU): x (N, cin, D, H, W) BF16 channels-last, w (cout, 27, cin) BF16."""
-    return _forward(x, w.contiguous(), w.shape[0], bias, relu)
+    return _forward(x, _aligned(w.contiguous()), w.shape[0], bias, relu)
 
 
 def _forward(x, w, cout, bias, relu):
-    """conv3d_forward of weights that are contiguous, in whatever shape."""
+    """conv3d_forward of weights that are contiguous and aligned, in whatever shape."""
     lib = _lib()
-    x, w = _volume(x), _aligned(w)
+    x = _volume(x)
     n, cin, d, h, wd = x.shape
     y = torch.empty((n, cout, d, h, wd), device=x.device, dtype=torch.bfloat16, memory_format=torch.channels_last_3d)
     b = bias.contiguous().float() if bias is not None else None
@@ -152,7 +153,7 @@ class Conv3dFunction(torch.autograd.Function):
     def forward(ctx, x, weight, bias, relu, packed=None):
         if packed is None:
             pairs = pack_weights([weight], [ctx.needs_input_grad[0]])
-            packed = pairs[0] if pairs else (weight.to(torch.bfloat16).contiguous(), None)
+            packed = pairs[0] if pairs else (_aligned(weight.to(torch.bfloat16).contiguous()), None)
         w16, wt = packed
         y = _forward(x, w16, weight.shape[0], bias, relu)
         ctx.save_for_backward(x, w16, wt, y if relu else None)
@@ -165,7 +166,7 @@ class Conv3dFunction(torch.autograd.Function):
         dy, db = relu_bias_grad(dy, y)
         dx = None
         if ctx.needs_input_grad[0]:
-            dx = (_forward(dy, wt.contiguous(), ctx.shape[2], None, False) if wt is not None
+            dx = (_forward(dy, _aligned(wt.contiguous()), ctx.shape[2], None, False) if wt is not None
                   else conv3d_input_grad(dy, w16.view(ctx.shape)))
         dw = conv3d_weight_grad(x, dy)
         return dx, dw, db, None, None
@@ -176,6 +177,12 @@ def _empty_volume(like, channels, d, h, w):
                        memory_format=torch.channels_last_3d)
 
 
+@functools.lru_cache(maxsize=256)
+def _bias_scratch(voxels, channels):
+    """Bytes of scratch of the bias's gradient."""
+    return _lib().lbm_net_relu_bias_scratch(voxels, channels)
+
+
 def relu_bias_grad(dy, y=None):
     """The gradient of a convolution's output before its ReLU (y, the layer's output; None without one), in BF16, and
     its sums over the voxels in FP32: the bias's gradient."""
@@ -184,7 +191,7 @@ def relu_bias_grad(dy, y=None):
     channels = dy.shape[1]
     voxels = dy.numel()//channels
     db = torch.empty(channels, device=dy.device, dtype=torch.float32)
-    scratch = torch.empty(lib.lbm_net_relu_bias_scratch(voxels, channels), device=dy.device, dtype=torch.uint8)
+    scratch = torch.empty(_bias_scratch(voxels, channels), device=dy.device, dtype=torch.uint8)
     out = dy
     if y is not None:
         y = _volume(y)
