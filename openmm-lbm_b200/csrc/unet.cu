@@ -796,7 +796,7 @@ convForwardKernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __re
 // (all dz of an MMA, or one) that are read and cleared while the next unit fills.
 //
 // Bound: 16 -> 16 channels read 4 KB of x and 4.6 KB of dy (68 wavefronts of shared memory) per MMA and 16 voxels, 19 us
-// on two 64 x 64 x 128 volumes.  Measured there: 79 us, what remains being the copies (dy three times) and the atomics of
+// on two 64 x 64 x 128 volumes.  Measured there: 76 us, what remains being the copies (dy three times) and the atomics of
 // the finished sums (a quarter less, with an error of 4e-6 instead of 9e-7, when a CTA adds its sums once); 1150 us with
 // the kernel before it, which gathered both operands transposed element by element and waited for each stage.  48 -> 16:
 // 160 us (4000), 32 -> 32 at 32 x 32 x 64 29 us (314), 160 -> 160 at 8 x 8 x 16 25 us (116).
